@@ -4,9 +4,14 @@
  * HBM layout of one field (one float32 array per field per component):
  *   x fastest, then y, then z;  element (i,j,k) of the Fortran index space
  *   (i = -1..nx+2, j = -1..ny+2, k = -1..nz+2, k = nz the free surface) lives
- *   at  (k+1)*plane + (j+1)*px + (i + XO - 1)  with XO = 8, so that x = 1
- *   starts on a 32-byte sector and every row of px floats is 32-byte aligned.
- *   px = round_up(nx + XO + 2, 8), plane = px * (ny + 4).
+ *   at  (k+1)*plane + (j+1)*px + (i + XO - 1)  with XO = 8.
+ *   px = round_up(nx + XO + 2, 32), plane = px * (ny + 4), and the arrays'
+ *   base addresses are placed so that x = 1 starts a 128-byte line in every
+ *   row: the 32-cell row of a tile is then one line, read and written whole.
+ *   (With x = 1 on a 32-byte sector only, every tile row straddled two lines
+ *   shared with the neighbouring tile, and what a tile left of them was
+ *   fetched again once the blocks drifted apart.)  A grid whose padded rows
+ *   would exceed the 32-bit index range keeps rows of a multiple of 8 floats.
  * Ghost cells hold zeros for wavefields (the boundary values of a single
  * domain), the padded values of padmedia/afsmedia for media.
  */

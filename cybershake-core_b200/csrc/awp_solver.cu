@@ -58,6 +58,8 @@ static awp_status set_err(awp_status st, const char *fmt, ...)
                            "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__);   \
     } while (0)
 
+#define AWP_MAX_FIELDS 128
+
 struct awp_solver {
     awp_params p;
     AwpGeom g;
@@ -93,7 +95,7 @@ struct awp_solver {
     float *kin[AWP_MAX_COMP];        /* kinematic subfault increments       */
     size_t stagger;                  /* base-address offset step of the field arrays */
     int nstag;
-    struct { void *user, *raw; } stag[128];
+    struct { void *user, *raw; } stag[AWP_MAX_FIELDS];   /* field arrays: pointer in use, block */
     int kchunk_staged;               /* z levels per staged work item       */
     int staged_qslow;                /* staged items: component slowest     */
     int staged_rpt;                  /* staged stress sweep rows per thread */
@@ -178,7 +180,8 @@ static AwpGeom make_geom(const awp_params *p)
 {
     AwpGeom g;
     g.nx = p->nx; g.ny = p->ny; g.nz = p->nz;
-    g.px = ((p->nx + AWP_XO + 2) + 7) / 8 * 8;
+    g.px = ((p->nx + AWP_XO + 2) + 31) / 32 * 32;
+    if ((int64_t)g.px * (p->ny + 4) * (p->nz + 4) >= (int64_t)1 << 31) g.px = ((p->nx + AWP_XO + 2) + 7) / 8 * 8;
     g.py = p->ny + 4;
     g.plane = g.px * g.py;
     g.vol = (int64_t)g.plane * (p->nz + 4);
@@ -477,20 +480,24 @@ static awp_status dalloc(awp_solver *s, void **ptr, size_t bytes)
     return AWP_OK;
 }
 
-/* field arrays with staggered base addresses (AWP_TUNE_STAGGER bytes times the
- * array's ordinal, modulo 32 ordinals), so that the same cell of different
- * arrays does not always fall on the same DRAM channel */
-static awp_status dalloc_field(awp_solver *s, void **ptr, size_t bytes)
+/* Field arrays.  x = 1 sits at column 8 of a row; the base is placed so that
+ * this column starts a 128-byte line (rows are a multiple of 128 bytes,
+ * make_geom), so the 32-cell row of a tile is one line of its own instead of
+ * parts of two that the neighbouring tile shares.  AWP_TUNE_STAGGER adds that
+ * many bytes times the array's ordinal (modulo 32). */
+static awp_status dalloc_field(awp_solver *s, void **ptr, size_t bytes, int esize)
 {
-    const size_t off = s->stagger * (size_t)(s->nstag % 32);
+    const size_t shift = (size_t)(128 - AWP_XO * esize), off = s->stagger * (size_t)(s->nstag % 32) + shift;
     void *raw = NULL;
     awp_status st = dalloc(s, &raw, bytes + off);
     if (st != AWP_OK) return st;
-    *ptr = (char *)raw + off;
-    if (off && s->nstag < 128) {
-        s->stag[s->nstag].user = *ptr;
-        s->stag[s->nstag].raw = raw;
-    }
+    *ptr = raw;
+    for (int n = 0; n < AWP_MAX_FIELDS; n++)
+        if (!s->stag[n].raw) {
+            *ptr = s->stag[n].user = (char *)raw + off;
+            s->stag[n].raw = raw;
+            break;
+        }
     s->nstag++;
     return AWP_OK;
 }
@@ -498,8 +505,8 @@ static awp_status dalloc_field(awp_solver *s, void **ptr, size_t bytes)
 static void dfree_field(awp_solver *s, void *p)
 {
     if (!p) return;
-    for (int n = 0; n < s->nstag && n < 128; n++)
-        if (s->stag[n].user == p && s->stag[n].raw) {
+    for (int n = 0; n < AWP_MAX_FIELDS; n++)
+        if (s->stag[n].raw && s->stag[n].user == p) {
             dfree(s, s->stag[n].raw);
             s->stag[n].raw = NULL;
             return;
@@ -553,7 +560,7 @@ static awp_status alloc_media32(awp_solver *s)
     const size_t vb = (size_t)s->g.vol * sizeof(float);
     for (int m = 0; m < AM_N; m++) {
         if (s->md.m[m]) continue;
-        awp_status st = dalloc_field(s, (void **)&s->md.m[m], vb);
+        awp_status st = dalloc_field(s, (void **)&s->md.m[m], vb, 4);
         if (st != AWP_OK) return st;
         CU(cudaMemsetAsync(s->md.m[m], 0, vb, s->stream));
         if (s->store == AWP_STORE_F32) s->mdt.m[m] = s->md.m[m];
@@ -599,15 +606,15 @@ extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
         for (int f = 0; f < AWP_NF_ARRAYS; f++) {
             if (f >= AF_R1) {
                 if (p->nve == 0 || (f == AF_RX && s->rstore != AWP_STORE_BFP)) continue;
-                TRY(dalloc_field(s, (void **)&s->comp[0][q].f[f], rb));
+                TRY(dalloc_field(s, (void **)&s->comp[0][q].f[f], rb, s->rstore == AWP_STORE_F32 ? 4 : 2));
                 TRYCU(cudaMemsetAsync(s->comp[0][q].f[f], 0, rb, s->stream));
                 s->comp[1][q].f[f] = s->comp[0][q].f[f];
                 continue;
             }
-            TRY(dalloc_field(s, (void **)&s->comp[0][q].f[f], vb));
+            TRY(dalloc_field(s, (void **)&s->comp[0][q].f[f], vb, 4));
             TRYCU(cudaMemsetAsync(s->comp[0][q].f[f], 0, vb, s->stream));
             if (s->fused) {
-                TRY(dalloc_field(s, (void **)&s->comp[1][q].f[f], vb));
+                TRY(dalloc_field(s, (void **)&s->comp[1][q].f[f], vb, 4));
                 TRYCU(cudaMemsetAsync(s->comp[1][q].f[f], 0, vb, s->stream));
             } else {
                 s->comp[1][q].f[f] = s->comp[0][q].f[f];
