@@ -52,13 +52,10 @@ struct AwpStepArgs {
     int kchunk_staged;           /* z levels per staged work item           */
     int staged_qslow;            /* staged items: one component at a time   */
     int staged_rpt;              /* staged stress sweep: tile rows per thread */
-    int staged_rpt_vel;          /* staged velocity sweep: tile rows per thread */
-    int staged_batch;            /* staged sweeps with the components side by side in one item:
-                                    bit 0 stress, bit 1 velocity */
+    int staged_batch;            /* bit 0: staged stress sweep with the components side by side in one item */
     int *kerr;                   /* device error word (AWP_KERR_*)          */
     int sm_limit;                /* persistent grids sized for this many SMs (0 = all) */
     int fma;                     /* staged sweeps compiled with multiply-add contraction */
-    int staged_generic;          /* one-component staged sweeps read their rings with generic loads */
     const AwpPmlArgs *pml;       /* NPC = 1: the PML zones after each sweep (NULL: Cerjan) */
     unsigned long long wait_ns;  /* bound of one barrier wait of the staged sweeps */
     int withhold;                /* test injection, -1 = off: block 0's producer of the

@@ -101,7 +101,6 @@ struct awp_solver {
     int staged_rpt;                  /* staged stress sweep rows per thread */
     int staged_rpt_vel;              /* staged velocity sweep rows per thread */
     int staged_batch;                /* staged stress: components in one item */
-    int staged_generic;              /* staged one-component sweeps: generic ring loads */
     int sm_limit;                    /* persistent grids for this many SMs (0 = all) */
     int fma;                         /* staged sweeps with multiply-add contraction */
     /* PML (npc = 1): split arrays per component, damping profiles, kernel arguments */
@@ -723,9 +722,6 @@ extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
          * so by default up to 32 GiB of solver state */
         const int batch_default = (double)awp_footprint_bytes(p, 0) <= 32.0 * (double)(1ull << 30) ? 1 : 0;
         s->staged_batch = env_int("AWP_TUNE_BATCH", batch_default) & 3;
-        /* the one-component sweeps read their rings with generic loads above
-         * 32 GiB of state, where that measured faster (awp_staged.cu) */
-        s->staged_generic = env_int("AWP_TUNE_GENERIC", batch_default ? 0 : 1) != 0;
     }
     s->nt_file = nt_file_of(p);
     s->nsamp_written = ((p->nt / p->ntiskp_sgt) / p->write_step) * p->write_step;
@@ -1220,9 +1216,7 @@ static void fill_args(awp_solver *s, int steps, AwpStepArgs &a, AwpPostArgs &pa,
     a.kchunk_staged = s->kchunk_staged;
     a.staged_qslow = s->staged_qslow;
     a.staged_rpt = s->staged_rpt;
-    a.staged_rpt_vel = s->staged_rpt_vel;
     a.staged_batch = s->staged_batch;
-    a.staged_generic = s->staged_generic;
     a.sm_limit = s->sm_limit;
     a.fma = s->fma;
     a.pml = s->p.npc == 1 ? &s->pml_args : NULL;
@@ -1489,9 +1483,8 @@ extern "C" awp_status awp_profile_steps(awp_solver *s, int nsteps, awp_kernel_ti
     o->nkernels = nk;
     for (int k = 0; k < np; k++) {
         const bool bstr = s->staged_on && parts[k] == AWP_PART_STR && (s->staged_batch & 1) && p->ncomp >= 2;
-        const bool bvel = s->staged_on && parts[k] == AWP_PART_VEL && (s->staged_batch & 2) && p->ncomp >= 2;
         snprintf(o->name[k], sizeof o->name[k], "%s",
-                 bstr ? "k_str_tmab" : (bvel ? "k_vel_tmab" : (s->staged_on ? pname_staged : pname)[parts[k]]));
+                 bstr ? "k_str_tmab" : (s->staged_on ? pname_staged : pname)[parts[k]]);
         o->bytes_per_launch[k] = part_bytes(s, parts[k]);
     }
     snprintf(o->name[np], sizeof o->name[np], "k_post");
@@ -2362,12 +2355,11 @@ extern "C" awp_status awp_autotune(const awp_params *pin, const float *media, in
     double cur_rate = 0.0;
     if (st == AWP_OK) st = tune_trial(s, &cur, trial_steps, &cur_rate);
     /* coordinate descent over the fields the stepper uses */
-    enum { F_KSTAGE, F_RPT, F_UNROLL, F_QSLOW, F_RPTV, F_TY, F_KFUSED, F_KSWEEP, F_BATCH };
-    int fields[9], nf = 0;
+    enum { F_KSTAGE, F_RPT, F_UNROLL, F_QSLOW, F_TY, F_KFUSED, F_KSWEEP, F_BATCH };
+    int fields[8], nf = 0;
     if (stepper == AWP_KERNEL_STAGED || stepper == AWP_KERNEL_STAGED_FMA) {
         if (p.ncomp >= 2) fields[nf++] = F_BATCH;
         fields[nf++] = F_KSTAGE, fields[nf++] = F_RPT, fields[nf++] = F_UNROLL, fields[nf++] = F_QSLOW;
-        fields[nf++] = F_RPTV;
     } else if (stepper == AWP_KERNEL_FUSED) {
         fields[nf++] = F_TY, fields[nf++] = F_KFUSED;
     } else {
@@ -2391,17 +2383,9 @@ extern "C" awp_status awp_autotune(const awp_params *pin, const float *media, in
         case F_RPT:
             if (!((cur.staged_batch & 1) && p.ncomp >= 2)) vals[nv++] = 3 - cur.staged_rpt;
             break;
-        case F_RPTV:
-            if (!((cur.staged_batch & 2) && p.ncomp >= 2)) vals[nv++] = 3 - cur.staged_rpt_vel;
-            break;
         case F_UNROLL: vals[nv++] = 3 - cur.unroll; break;
-        case F_QSLOW:
-            if (!(cur.staged_batch == 3 && p.ncomp >= 2)) vals[nv++] = 1 - cur.staged_qslow;
-            break;
-        case F_BATCH:
-            for (int b = 0; b < 4; b++)
-                if (b != cur.staged_batch) vals[nv++] = b;
-            break;
+        case F_QSLOW: vals[nv++] = 1 - cur.staged_qslow; break;
+        case F_BATCH: vals[nv++] = cur.staged_batch ^ 1; break;
         case F_TY:
             for (int ty : {4, 8, 16})
                 if (ty != cur.ty && (stepper == AWP_KERNEL_FUSED || ty != 16)) vals[nv++] = ty;
@@ -2420,7 +2404,6 @@ extern "C" awp_status awp_autotune(const awp_params *pin, const float *media, in
             switch (fields[fi]) {
             case F_KSTAGE: cand.kchunk_staged = vals[vi]; break;
             case F_RPT: cand.staged_rpt = vals[vi]; break;
-            case F_RPTV: cand.staged_rpt_vel = vals[vi]; break;
             case F_UNROLL: cand.unroll = vals[vi]; break;
             case F_QSLOW: cand.staged_qslow = vals[vi]; break;
             case F_BATCH: cand.staged_batch = vals[vi]; break;

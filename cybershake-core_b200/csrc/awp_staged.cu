@@ -1,8 +1,8 @@
 /*
  * awp_staged.cu -- the two-sweep stepper with TMA-staged xy tiles (2.5D blocking).
  *
- * A thread block owns a 32 x 8 column tile of one component and marches up a
- * chunk of z levels.  A producer warp issues, for every level, TMA tile loads
+ * A thread block owns a 32 x 8 column tile (the velocity sweep, awp_pair.cuh:
+ * 32 x 16) of one component and marches up a chunk of z levels.  A producer warp issues, for every level, TMA tile loads
  * (cp.async.bulk.tensor over 3D tensor maps of the padded volume) into a ring
  * of shared-memory slots ahead of the level being computed: stencil tiles
  * with a 4-column and 2-row halo, media tiles with the row below, and the
@@ -52,13 +52,7 @@ struct AwpWait {
     unsigned long long ns;
     int withhold;
 };
-#define ST_VEL_D 3                   /* levels in flight, velocity sweep        */
 
-struct AwpStagedVelMaps {
-    CUtensorMap st[AWP_MAX_COMP][5]; /* xx yy xy xz yz, box 40 x 12           */
-    CUtensorMap d1;                  /* box 40 x 9                             */
-    CUtensorMap p[AWP_MAX_COMP][3];  /* u v w, box 32 x 8                      */
-};
 struct AwpStagedStrMaps {
     CUtensorMap v[AWP_MAX_COMP][3];  /* u v w, box 40 x 12                     */
     CUtensorMap med[4];              /* lam mu qp qs, box 40 x 9               */
@@ -66,9 +60,21 @@ struct AwpStagedStrMaps {
     CUtensorMap r[AWP_MAX_COMP][6];  /* r1..r6 (FP32, bf16 or int16), box 32 x 8 */
     CUtensorMap rx[AWP_MAX_COMP];    /* exponent words of block floating point r */
 };
+/* tensor maps of the velocity sweep with two cells per thread (awp_pair.cuh) */
+struct AwpStagedVelMaps {
+    CUtensorMap xx[AWP_MAX_COMP];     /* box 40 x rows                           */
+    CUtensorMap yy[AWP_MAX_COMP];     /* box 32 x (rows + 3)                     */
+    CUtensorMap xy[AWP_MAX_COMP];     /* box 40 x (rows + 3)                     */
+    CUtensorMap xz[AWP_MAX_COMP];     /* box 40 x rows                           */
+    CUtensorMap yz[AWP_MAX_COMP];     /* box 32 x (rows + 3)                     */
+    CUtensorMap d1;                   /* box W x (rows + 1)                      */
+    CUtensorMap p[AWP_MAX_COMP][6];   /* u v w (plane k), zz xz yz (planes k+2 k+1 k+1), box 32 x rows */
+};
+#define PR_VEL_CW 8                  /* its consumer warps                      */
+
 struct AwpStaged {
-    AwpStagedVelMaps vm;
     AwpStagedStrMaps sm;
+    AwpStagedVelMaps vm;
 };
 
 /* The kernels live in an anonymous namespace: this file is compiled twice,
@@ -201,20 +207,6 @@ __device__ __forceinline__ float *ring_base(unsigned char *raw)
     return (float *)(raw + pad);
 }
 
-/* GL: the same address through an integer, so that the compiler reads the
- * ring with generic loads.  On the 1400 x 1000 x 400 workload (78 GB of
- * state, one component per work item) the sweeps ran faster that way:
- * 28.7 against 24.4 Gcell-updates/s on one box, velocity sweep 12.3 against
- * 14.3 ms and stress sweep 26.1 against 31.6 ms per launch, while on the 6.4
- * and 14.7 GB workloads shared-memory loads are 5-8 % faster.  The cause is
- * not known; the solver picks GL above 32 GiB of state (AWP_TUNE_GENERIC). */
-template <bool GL>
-__device__ __forceinline__ float *ring_base_t(unsigned char *raw)
-{
-    if (GL) return (float *)(((uintptr_t)raw + 127) & ~(uintptr_t)127);
-    return ring_base(raw);
-}
-
 template <int S>
 __device__ __forceinline__ void ring_init(uint64_t *full, uint64_t *empty, volatile int *abort, int consumers = ST_CW)
 {
@@ -251,331 +243,6 @@ __device__ __forceinline__ bool ring_acquire(uint64_t *empty, uint32_t use, cons
                                              uint64_t limit_ns)
 {
     return use < (uint32_t)S || mb_wait_or_abort(&empty[use % S], ((use / S) - 1) & 1, abort, limit_ns);
-}
-
-/* ------------------------------------------------------------------ */
-/* velocity sweep                                                      */
-/* ------------------------------------------------------------------ */
-
-/* slot layout: xx yy xy xz yz stencil tiles, the d1 media tile, then the
- * u v w point tiles */
-#define VEL_PT (5 * ST_VT + ST_MP)
-#define VEL_SLOT (VEL_PT + 3 * ST_PT)
-#define VEL_TXB ((5 * ST_VT + ST_MT + 3 * ST_PT) * 4)
-
-/* stresses of plane k from the slot (in-plane) and from the register queue (z) */
-struct TStr {
-    const float *t; /* slot + cell offset */
-    float xz_m2, xz_m1, xz_p1, yz_m2, yz_m1, yz_p1, zz_m1, zz_0, zz_p1, zz_p2;
-    __device__ __forceinline__ float s(int a, int dx, int dy, int dz) const
-    {
-        if (a == S_ZZ) return dz == -1 ? zz_m1 : (dz == 0 ? zz_0 : (dz == 1 ? zz_p1 : zz_p2));
-        if (dz == 0) {
-            const int n = a == S_XX ? 0 : (a == S_YY ? 1 : (a == S_XY ? 2 : (a == S_XZ ? 3 : 4)));
-            return t[n * ST_VT + dy * ST_W + dx];
-        }
-        if (a == S_XZ) return dz == -2 ? xz_m2 : (dz == -1 ? xz_m1 : xz_p1);
-        return dz == -2 ? yz_m2 : (dz == -1 ? yz_m1 : yz_p1);
-    }
-};
-
-template <int S>
-__device__ __forceinline__ void vel_issue(const CUtensorMap *ms, const CUtensorMap *md1, const CUtensorMap *mp,
-                                          float *ring, uint64_t *full, uint32_t use, int i0, int j0, int k)
-{
-    float *sl = ring + (use % S) * VEL_SLOT;
-    uint64_t *b = &full[use % S];
-    fence_async_smem();
-    mb_expect(b, VEL_TXB);
-    const int x = tile_x(i0);
-#pragma unroll
-    for (int a = 0; a < 5; ++a) tma_3d(sl + a * ST_VT, ms + a, b, x, j0 - 1, k + 1);
-    tma_3d(sl + 5 * ST_VT, md1, b, x, j0, k + 1);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) tma_3d(sl + VEL_PT + a * ST_PT, mp + a, b, i0 + AWP_XO - 1, j0 + 1, k + 1);
-}
-
-/* work items: (x tile, y tile, z chunk, component); see split_item for the order */
-template <int D, int UNR, int RPT, bool GL = false>
-__global__ void __launch_bounds__(32 * (ST_Y / RPT + 1), 3)
-k_vel_tma(const __grid_constant__ AwpStagedVelMaps maps, AwpGeom g, AwpCompSet<AWP_MAX_COMP> cs, int ncomp, int qslow,
-          const float *__restrict__ d1, const float *__restrict__ cx, const float *__restrict__ cy,
-          const float *__restrict__ cz, float dth, AwpWork w, int *err, AwpWait wt)
-{
-    constexpr int S = 1 + D;          /* level k in use, D in flight */
-    constexpr int CW = ST_Y / RPT;    /* consumer warps */
-    extern __shared__ unsigned char st_smem[];
-    float *ring = ring_base_t<GL>(st_smem);
-    uint64_t *full = (uint64_t *)(ring + S * VEL_SLOT), *empty = full + S;
-    __shared__ volatile int abort_s;
-    ring_init<S>(full, empty, &abort_s, CW);
-    const int tx = threadIdx.x, ty = threadIdx.y;
-
-    if (ty == CW) {                   /* producer warp */
-        if (tx != 0) return;
-        uint32_t use = 0;
-        bool ok = true;
-        for (int item = blockIdx.x; ok && item < w.nitems; item += gridDim.x) {
-            int q, t;
-            split_item(item, ncomp, w.nitems / ncomp, qslow, q, t);
-            int bx, by, k0, k1;
-            work_item(g, w, t, bx, by, k0, k1);
-            for (int k = k0; k <= k1; ++k, ++use) {
-                ok = ring_acquire<S>(empty, use, &abort_s, wt.ns);
-                if (!ok) break;
-                vel_issue<S>(maps.st[q], &maps.d1, maps.p[q], ring, full, use, bx * ST_X + 1, by * ST_Y + 1, k);
-            }
-        }
-        if (!ok) {
-            abort_s = 1;
-            atomicOr(err, AWP_KERR_TMA_WAIT);
-        }
-        ring_drain<S>(full, use, wt.ns);
-        return;
-    }
-
-    const int sy = g.px, sz = g.plane;
-    uint32_t use = 0;
-    for (int item = blockIdx.x; item < w.nitems; item += gridDim.x) {
-        int q, t;
-        split_item(item, ncomp, w.nitems / ncomp, qslow, q, t);
-        int bx, by, k0, k1;
-        work_item(g, w, t, bx, by, k0, k1);
-        const int i = bx * ST_X + 1 + tx;
-        float *U = pick(cs, q, AF_U), *V = pick(cs, q, AF_V), *W = pick(cs, q, AF_W);
-        const float *XZ = pick(cs, q, AF_XZ), *YZ = pick(cs, q, AF_YZ), *ZZ = pick(cs, q, AF_ZZ);
-        /* per row: column queues, each loaded one level before it is needed */
-        float xz_m2[RPT], xz_m1[RPT], xz_p1[RPT], yz_m2[RPT], yz_m1[RPT], yz_p1[RPT];
-        float zz_m1[RPT], zz_0[RPT], zz_p1[RPT], zz_p2[RPT], dA[RPT], dB[RPT], dE[RPT], cxy[RPT];
-        bool live[RPT];
-        const int c0 = g.idx(i, by * ST_Y + 1 + ty, k0);
-#pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-            const int j = by * ST_Y + 1 + ty + r * CW, c = c0 + r * CW * sy;
-            live[r] = i <= g.nx && j <= g.ny;
-            xz_m2[r] = xz_m1[r] = xz_p1[r] = yz_m2[r] = yz_m1[r] = yz_p1[r] = 0.f;
-            zz_m1[r] = zz_0[r] = zz_p1[r] = zz_p2[r] = dA[r] = dB[r] = dE[r] = cxy[r] = 0.f;
-            if (live[r]) {
-                xz_m2[r] = XZ[c - 2 * sz]; xz_m1[r] = XZ[c - sz]; xz_p1[r] = XZ[c + sz];
-                yz_m2[r] = YZ[c - 2 * sz]; yz_m1[r] = YZ[c - sz]; yz_p1[r] = YZ[c + sz];
-                zz_m1[r] = ZZ[c - sz]; zz_0[r] = ZZ[c]; zz_p1[r] = ZZ[c + sz]; zz_p2[r] = ZZ[c + 2 * sz];
-                dA[r] = d1[c - sz]; dB[r] = d1[c - sy - sz]; dE[r] = d1[c + 1 - sz];
-                cxy[r] = cx[i] * cy[j];
-            }
-        }
-        int cc = c0;
-#pragma unroll (UNR)
-        for (int k = k0; k <= k1; ++k, cc += sz, ++use) {
-            float xz_n[RPT], yz_n[RPT], zz_n[RPT];
-            const float czk = cz[k];
-#pragma unroll
-            for (int r = 0; r < RPT; ++r) {
-                const int c = cc + r * CW * sy;
-                xz_n[r] = yz_n[r] = zz_n[r] = 0.f;
-                if (live[r] && k < k1) { xz_n[r] = XZ[c + 2 * sz]; yz_n[r] = YZ[c + 2 * sz]; zz_n[r] = ZZ[c + 3 * sz]; }
-            }
-            /* warp-uniform outcome, so a warp leaves together or not at all */
-            if (!__all_sync(0xffffffffu, mb_wait_or_abort(&full[use % S], (use / S) & 1, &abort_s, wt.ns))) {
-                abort_s = 1;
-                atomicOr(err, AWP_KERR_TMA_WAIT);
-                return;
-            }
-            const float *sl = ring + (use % S) * VEL_SLOT;
-#pragma unroll
-            for (int r = 0; r < RPT; ++r) {
-                const int row = ty + r * CW, c = cc + r * CW * sy;
-                const int cv = (row + 2) * ST_W + tx + 4, cm = (row + 1) * ST_W + tx + 4, cp = row * ST_X + tx;
-                if (live[r]) {
-                    const float u0 = sl[VEL_PT + cp], v0 = sl[VEL_PT + ST_PT + cp], w0 = sl[VEL_PT + 2 * ST_PT + cp];
-                    const float *t1 = sl + 5 * ST_VT + cm;
-                    const float da = t1[0], db = t1[-ST_W], de = t1[1], dg = t1[1 - ST_W];
-                    float fu, fv, fw;
-                    vel_factors7(da, db, dA[r], dB[r], de, dE[r], dg, dth, fu, fv, fw);
-                    const TStr A{sl + cv, xz_m2[r], xz_m1[r], xz_p1[r], yz_m2[r], yz_m1[r], yz_p1[r],
-                                 zz_m1[r], zz_0[r], zz_p1[r], zz_p2[r]};
-                    float u, v, w_;
-                    vel_one_t(A, u0, v0, w0, fu, fv, fw, u, v, w_);
-                    const float crj = cxy[r] * czk;
-                    U[c] = u * crj;
-                    V[c] = v * crj;
-                    W[c] = w_ * crj;
-                    xz_m2[r] = xz_m1[r]; xz_m1[r] = sl[3 * ST_VT + cv];
-                    yz_m2[r] = yz_m1[r]; yz_m1[r] = sl[4 * ST_VT + cv];
-                    zz_m1[r] = zz_0[r]; zz_0[r] = zz_p1[r]; zz_p1[r] = zz_p2[r]; zz_p2[r] = zz_n[r];
-                    xz_p1[r] = xz_n[r]; yz_p1[r] = yz_n[r];
-                    dA[r] = da; dB[r] = db; dE[r] = de;
-                }
-            }
-            __syncwarp();
-            if (tx == 0) mb_arrive(&empty[use % S]);
-        }
-    }
-}
-
-/* ---- velocity sweep, components side by side ---------------------------- */
-
-/* One work item per (x tile, y tile, z chunk) for every component.  The d1
- * tile of a level comes once into a small ring of its own and the three
- * density factors of the cell are computed once for all components (plane
- * k-1 of d1 travels in registers); each component's stress stencil tiles and
- * u v w point tiles follow in a ring of sub-slots, one per (level,
- * component).  Column loads of the stresses are issued a full level before
- * they rotate in. */
-#define VB_MS 3                                   /* d1 slots                */
-#define VB_CPT (5 * ST_VT)                        /* first point tile        */
-#define VB_CSLOT (VB_CPT + 3 * ST_PT)
-
-template <int NCB, int CS>
-__global__ void __launch_bounds__(ST_THREADS, 2)
-k_vel_tmab(const __grid_constant__ AwpStagedVelMaps maps, AwpGeom g, AwpCompSet<AWP_MAX_COMP> cs,
-           const float *__restrict__ d1, const float *__restrict__ cx, const float *__restrict__ cy,
-           const float *__restrict__ cz, float dth, AwpWork w, int *err, AwpWait wt)
-{
-    extern __shared__ unsigned char st_smem[];
-    float *mring = ring_base(st_smem);
-    float *cring = mring + VB_MS * ST_MP;
-    uint64_t *mfull = (uint64_t *)(cring + CS * VB_CSLOT), *mempty = mfull + VB_MS;
-    uint64_t *cfull = mempty + VB_MS, *cempty = cfull + CS;
-    __shared__ volatile int abort_s;
-    __shared__ AwpComp tab[AWP_MAX_COMP];
-    if (threadIdx.y == 0 && threadIdx.x < AWP_MAX_COMP) {
-#pragma unroll
-        for (int f = 0; f < AWP_NF_ARRAYS; ++f) tab[threadIdx.x].f[f] = pick(cs, threadIdx.x, f);
-    }
-    ring_init<VB_MS>(mfull, mempty, &abort_s, ST_CW);
-    ring_init<CS>(cfull, cempty, &abort_s, ST_CW);
-    const int tx = threadIdx.x, ty = threadIdx.y;
-
-    if (ty == ST_CW) {                /* producer warp */
-        if (tx != 0) return;
-        uint32_t um = 0, uc = 0;
-        bool ok = true;
-        for (int item = blockIdx.x; ok && item < w.nitems; item += gridDim.x) {
-            int bx, by, k0, k1;
-            work_item(g, w, item, bx, by, k0, k1);
-            const int i0 = bx * ST_X + 1, j0 = by * ST_Y + 1;
-            const int x = tile_x(i0), xp = i0 + AWP_XO - 1;
-            for (int k = k0; ok && k <= k1; ++k) {
-                ok = ring_acquire<VB_MS>(mempty, um, &abort_s, wt.ns);
-                if (!ok) break;
-                {
-                    float *sl = mring + (um % VB_MS) * ST_MP;
-                    uint64_t *b = &mfull[um % VB_MS];
-                    fence_async_smem();
-                    mb_expect(b, ST_MT * 4);
-                    tma_3d(sl, &maps.d1, b, x, j0, k + 1);
-                }
-                ++um;
-#pragma unroll
-                for (int q = 0; q < NCB; ++q) {
-                    ok = ring_acquire<CS>(cempty, uc, &abort_s, wt.ns);
-                    if (!ok) break;
-                    float *sl = cring + (uc % CS) * VB_CSLOT;
-                    uint64_t *b = &cfull[uc % CS];
-                    fence_async_smem();
-                    mb_expect(b, (5 * ST_VT + 3 * ST_PT) * 4);
-#pragma unroll
-                    for (int a = 0; a < 5; ++a) tma_3d(sl + a * ST_VT, &maps.st[q][a], b, x, j0 - 1, k + 1);
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) tma_3d(sl + VB_CPT + a * ST_PT, &maps.p[q][a], b, xp, j0 + 1, k + 1);
-                    ++uc;
-                }
-            }
-        }
-        if (!ok) {
-            abort_s = 1;
-            atomicOr(err, AWP_KERR_TMA_WAIT);
-        }
-        ring_drain<VB_MS>(mfull, um, wt.ns);
-        ring_drain<CS>(cfull, uc, wt.ns);
-        return;
-    }
-
-    const int sy = g.px, sz = g.plane;
-    const int cv = (ty + 2) * ST_W + tx + 4, cm = (ty + 1) * ST_W + tx + 4, cp = ty * ST_X + tx;
-    uint32_t um = 0, uc = 0;
-    for (int item = blockIdx.x; item < w.nitems; item += gridDim.x) {
-        int bx, by, k0, k1;
-        work_item(g, w, item, bx, by, k0, k1);
-        const int i = bx * ST_X + 1 + tx, j = by * ST_Y + 1 + ty;
-        const bool live = i <= g.nx && j <= g.ny;
-        const int c0 = g.idx(i, j, k0);
-        /* per component: stresses along the column (xz, yz at k-2, k-1 from
-         * earlier tiles, k+1 from the pending load; zz at k-1 .. k+2), the
-         * pending loads one level ahead (pxz, pyz, pzz) */
-        float xz_m2[NCB], xz_m1[NCB], xz_p1[NCB], yz_m2[NCB], yz_m1[NCB], yz_p1[NCB];
-        float zz_m1[NCB], zz_0[NCB], zz_p1[NCB], zz_p2[NCB], pxz[NCB], pyz[NCB], pzz[NCB];
-        float dA = 0.f, dB = 0.f, dE = 0.f;
-#pragma unroll
-        for (int q = 0; q < NCB; ++q) {
-            xz_m2[q] = xz_m1[q] = xz_p1[q] = yz_m2[q] = yz_m1[q] = yz_p1[q] = 0.f;
-            zz_m1[q] = zz_0[q] = zz_p1[q] = zz_p2[q] = pxz[q] = pyz[q] = pzz[q] = 0.f;
-            if (live) {
-                const float *XZ = tab[q].f[AF_XZ], *YZ = tab[q].f[AF_YZ], *ZZ = tab[q].f[AF_ZZ];
-                xz_m2[q] = XZ[c0 - 2 * sz]; xz_m1[q] = XZ[c0 - sz]; pxz[q] = XZ[c0 + sz];
-                yz_m2[q] = YZ[c0 - 2 * sz]; yz_m1[q] = YZ[c0 - sz]; pyz[q] = YZ[c0 + sz];
-                zz_0[q] = ZZ[c0 - sz]; zz_p1[q] = ZZ[c0]; zz_p2[q] = ZZ[c0 + sz]; pzz[q] = ZZ[c0 + 2 * sz];
-            }
-        }
-        if (live) {
-            dA = d1[c0 - sz];
-            dB = d1[c0 - sy - sz];
-            dE = d1[c0 + 1 - sz];
-        }
-        const float cxy = live ? cx[i] * cy[j] : 0.f;
-        int cc = c0;
-#pragma unroll 1
-        for (int k = k0; k <= k1; ++k, cc += sz, ++um) {
-            const float czk = cz[k];
-            if (!__all_sync(0xffffffffu, mb_wait_or_abort(&mfull[um % VB_MS], (um / VB_MS) & 1, &abort_s, wt.ns))) {
-                abort_s = 1;
-                atomicOr(err, AWP_KERR_TMA_WAIT);
-                return;
-            }
-            float fu, fv, fw;
-            {
-                const float *t1 = mring + (um % VB_MS) * ST_MP + cm;
-                const float da = t1[0], db = t1[-ST_W], de = t1[1], dg = t1[1 - ST_W];
-                vel_factors7(da, db, dA, dB, de, dE, dg, dth, fu, fv, fw);
-                dA = da; dB = db; dE = de;
-            }
-            __syncwarp();
-            if (tx == 0) mb_arrive(&mempty[um % VB_MS]);
-#pragma unroll
-            for (int q = 0; q < NCB; ++q, ++uc) {
-                zz_m1[q] = zz_0[q]; zz_0[q] = zz_p1[q]; zz_p1[q] = zz_p2[q]; zz_p2[q] = pzz[q];
-                xz_p1[q] = pxz[q]; yz_p1[q] = pyz[q];
-                pxz[q] = pyz[q] = pzz[q] = 0.f;
-                if (live && k < k1) {
-                    pxz[q] = tab[q].f[AF_XZ][cc + 2 * sz];
-                    pyz[q] = tab[q].f[AF_YZ][cc + 2 * sz];
-                    pzz[q] = tab[q].f[AF_ZZ][cc + 3 * sz];
-                }
-                if (!__all_sync(0xffffffffu, mb_wait_or_abort(&cfull[uc % CS], (uc / CS) & 1, &abort_s, wt.ns))) {
-                    abort_s = 1;
-                    atomicOr(err, AWP_KERR_TMA_WAIT);
-                    return;
-                }
-                const float *sl = cring + (uc % CS) * VB_CSLOT;
-                const float nxz = sl[3 * ST_VT + cv], nyz = sl[4 * ST_VT + cv];
-                if (live) {
-                    const float u0 = sl[VB_CPT + cp], v0 = sl[VB_CPT + ST_PT + cp], w0 = sl[VB_CPT + 2 * ST_PT + cp];
-                    const TStr A{sl + cv, xz_m2[q], xz_m1[q], xz_p1[q], yz_m2[q], yz_m1[q], yz_p1[q],
-                                 zz_m1[q], zz_0[q], zz_p1[q], zz_p2[q]};
-                    float u, v, w_;
-                    vel_one_t(A, u0, v0, w0, fu, fv, fw, u, v, w_);
-                    const float crj = cxy * czk;
-                    tab[q].f[AF_U][cc] = u * crj;
-                    tab[q].f[AF_V][cc] = v * crj;
-                    tab[q].f[AF_W][cc] = w_ * crj;
-                }
-                __syncwarp();
-                if (tx == 0) mb_arrive(&cempty[uc % CS]);
-                xz_m2[q] = xz_m1[q]; xz_m1[q] = nxz;
-                yz_m2[q] = yz_m1[q]; yz_m1[q] = nyz;
-            }
-        }
-    }
 }
 
 /* ------------------------------------------------------------------ */
@@ -686,7 +353,7 @@ __device__ __forceinline__ void str_issue(const AwpStagedStrMaps &maps, int q, i
 /* work items: (x tile, y tile, z chunk, component); see split_item for the order.
  * RPT rows of the tile per consumer thread (ST_Y / RPT consumer warps): with
  * RPT = 2 a thread carries two independent cells per level. */
-template <class TR, int UNR, int RPT, bool GL = false>
+template <class TR, int UNR, int RPT>
 __global__ void __launch_bounds__(32 * (ST_Y / RPT + 1), 3)
 k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<AWP_MAX_COMP> cs, int ncomp, int qslow,
           const float *__restrict__ cx, const float *__restrict__ cy, const float *__restrict__ cz,
@@ -695,7 +362,7 @@ k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<A
     constexpr int S = 2 + STR_D;      /* levels k-1 and k in use, STR_D in flight */
     constexpr int CW = ST_Y / RPT;    /* consumer warps */
     extern __shared__ unsigned char st_smem[];
-    float *ring = ring_base_t<GL>(st_smem);
+    float *ring = ring_base(st_smem);
     uint64_t *full = (uint64_t *)(ring + S * STR_SLOT), *empty = full + S;
     __shared__ volatile int abort_s;
     __shared__ AwpComp tab[AWP_MAX_COMP];
@@ -768,10 +435,7 @@ k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<A
             for (int r = 0; r < RPT; ++r) {
                 const int c = cc + r * CW * sy;
                 up3[r] = vp3[r] = wp2[r] = 0.f;
-                if (live[r] && k < k1) {
-                    if (GL) { up3[r] = U[c + 3 * sz]; vp3[r] = V[c + 3 * sz]; wp2[r] = W[c + 2 * sz]; }
-                    else { up3[r] = __ldg(&U[c + 3 * sz]); vp3[r] = __ldg(&V[c + 3 * sz]); wp2[r] = __ldg(&W[c + 2 * sz]); }
-                }
+                if (live[r] && k < k1) { up3[r] = __ldg(&U[c + 3 * sz]); vp3[r] = __ldg(&V[c + 3 * sz]); wp2[r] = __ldg(&W[c + 2 * sz]); }
             }
             bool ok = true;
             if (k == k0) ok = mb_wait_or_abort(&full[usem % S], (usem / S) & 1, &abort_s, wt.ns);
@@ -806,12 +470,7 @@ k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<A
                         o = str_elastic(kc, Vq, s0, dth);
                     }
                     const float crj = cxy[r] * czk;
-                    if (GL) {
-                        tab[q].f[AF_XX][c] = o.xx * crj; tab[q].f[AF_YY][c] = o.yy * crj; tab[q].f[AF_ZZ][c] = o.zz * crj;
-                        tab[q].f[AF_XY][c] = o.xy * crj; tab[q].f[AF_XZ][c] = o.xz * crj; tab[q].f[AF_YZ][c] = o.yz * crj;
-                    } else {
-                        gst6(tab[q], c, o, crj);
-                    }
+                    gst6(tab[q], c, o, crj);
                 }
                 up1[r] = up2[r]; up2[r] = up3[r];
                 vp1[r] = vp2[r]; vp2[r] = vp3[r];
@@ -1074,6 +733,8 @@ k_str_tmab(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<
     }
 }
 
+#include "awp_pair.cuh"
+
 }  // namespace
 
 /* ------------------------------------------------------------------ */
@@ -1128,13 +789,10 @@ cudaError_t awp_staged_create(AwpStaged **out, const AwpGeom &g, int ncomp, cons
     AwpStaged *s = (AwpStaged *)aligned_alloc(64, sizeof(AwpStaged));
     if (!s) return cudaErrorMemoryAllocation;
     memset(s, 0, sizeof *s);
-    static const int vel_f[5] = {AF_XX, AF_YY, AF_XY, AF_XZ, AF_YZ};
     static const int med_f[4] = {AM_LAM, AM_MU, AM_QP, AM_QS};
     const int rsize = rtype == AWP_STORE_F32 ? 4 : 2;
-    bool ok = make_map(&s->vm.d1, g, md.m[AM_D1], ST_W, ST_MR);
+    bool ok = true;
     for (int q = 0; q < ncomp; ++q) {
-        for (int a = 0; a < 5; ++a) ok = ok && make_map(&s->vm.st[q][a], g, comp[q].f[vel_f[a]], ST_W, ST_HR);
-        for (int a = 0; a < 3; ++a) ok = ok && make_map(&s->vm.p[q][a], g, comp[q].f[AF_U + a], ST_X, ST_Y);
         for (int a = 0; a < 3; ++a) ok = ok && make_map(&s->sm.v[q][a], g, comp[q].f[AF_U + a], ST_W, ST_HR);
         for (int a = 0; a < 6; ++a) ok = ok && make_map(&s->sm.s[q][a], g, comp[q].f[AF_XX + a], ST_X, ST_Y);
         for (int a = 0; a < 6; ++a)     /* absent in the elastic scheme, which never loads them */
@@ -1143,6 +801,16 @@ cudaError_t awp_staged_create(AwpStaged **out, const AwpGeom &g, int ncomp, cons
             ok = ok && comp[q].f[AF_RX] && make_map(&s->sm.rx[q], g, comp[q].f[AF_RX], ST_X, ST_Y, 2);
     }
     for (int a = 0; a < 4; ++a) ok = ok && make_map(&s->sm.med[a], g, md.m[med_f[a]], ST_W, ST_MR);
+    const int vr = 2 * PR_VEL_CW;
+    ok = ok && make_map(&s->vm.d1, g, md.m[AM_D1], MedRow<float>::W, vr + 1);
+    for (int q = 0; q < ncomp; ++q) {
+        const AwpComp &o = comp[q];
+        static const int pf[6] = {AF_U, AF_V, AF_W, AF_ZZ, AF_XZ, AF_YZ};
+        ok = ok && make_map(&s->vm.xx[q], g, o.f[AF_XX], PR_W, vr) && make_map(&s->vm.yy[q], g, o.f[AF_YY], PR_X, vr + 3) &&
+             make_map(&s->vm.xy[q], g, o.f[AF_XY], PR_W, vr + 3) && make_map(&s->vm.xz[q], g, o.f[AF_XZ], PR_W, vr) &&
+             make_map(&s->vm.yz[q], g, o.f[AF_YZ], PR_X, vr + 3);
+        for (int a = 0; a < 6; ++a) ok = ok && make_map(&s->vm.p[q][a], g, o.f[pf[a]], PR_X, vr);
+    }
     if (!ok) {
         free(s);
         return cudaErrorInvalidValue;
@@ -1196,33 +864,34 @@ static AwpCompSet<AWP_MAX_COMP> comp_set3(const AwpStepArgs &s)
     return cs;
 }
 
-/* dynamic shared memory of a ring: alignment slack, slots, full + empty barriers */
-static size_t ring_bytes(int slots, int slot_floats) { return 128 + (size_t)slots * slot_floats * 4 + 2 * 8 * slots; }
-
-template <int UNR>
-static cudaError_t launch_vel_u(const AwpStaged *st, const AwpStepArgs &s, cudaStream_t stream)
+static AwpWork pair_work(const AwpGeom &g, int rows, int kchunk, int ncomp)
 {
-    constexpr int RPT = UNR < 0 ? 2 : 1;            /* UNR -1: two rows per thread, level loop rolled */
-    constexpr int U = UNR < 0 ? 1 : UNR;
-    constexpr int CW = ST_Y / RPT;
-    const size_t smem = ring_bytes(1 + ST_VEL_D, VEL_SLOT);
-    const AwpWork w = staged_work(s.g, s.kchunk_staged, s.ncomp);
+    AwpWork w;
+    w.ntx = (g.nx + PR_X - 1) / PR_X;
+    w.nty = (g.ny + rows - 1) / rows;
+    w.kchunk = kchunk;
+    w.nzc = (g.nz + kchunk - 1) / kchunk;
+    w.nitems = w.ntx * w.nty * w.nzc * ncomp;
+    return w;
+}
+
+template <class TM>
+static cudaError_t launch_vel(const AwpStaged *st, const AwpStepArgs &s, cudaStream_t stream)
+{
+    constexpr int CW = PR_VEL_CW, S = 3;
+    const size_t smem = PairVelL<TM, CW>::smem(S);
+    const AwpWork w = pair_work(s.g, 2 * CW, s.kchunk_staged, s.ncomp);
     int grid = 0;
-    if (s.staged_generic && UNR == 2) {                 /* generic ring loads (ring_base_t) */
-        cudaError_t e = staged_grid(k_vel_tma<ST_VEL_D, 2, 1, true>, smem, w.nitems, &grid, s.sm_limit, 32 * (ST_Y + 1));
-        if (e != cudaSuccess) return e;
-        k_vel_tma<ST_VEL_D, 2, 1, true><<<grid, dim3(32, ST_Y + 1), smem, stream>>>(
-            st->vm, s.g, comp_set3(s), s.ncomp, s.staged_qslow, (const float *)s.md.m[AM_D1], s.cx, s.cy, s.cz, s.dth,
-            w, s.kerr, awp_wait_of(s));
-        return cudaGetLastError();
-    }
-    cudaError_t e = staged_grid(k_vel_tma<ST_VEL_D, U, RPT>, smem, w.nitems, &grid, s.sm_limit, 32 * (CW + 1));
+    cudaError_t e = staged_grid(k_vel_tma<TM, CW, S, 2>, smem, w.nitems, &grid, s.sm_limit, 32 * (CW + 1));
     if (e != cudaSuccess) return e;
-    k_vel_tma<ST_VEL_D, U, RPT><<<grid, dim3(32, CW + 1), smem, stream>>>(
-        st->vm, s.g, comp_set3(s), s.ncomp, s.staged_qslow, (const float *)s.md.m[AM_D1], s.cx, s.cy, s.cz, s.dth, w,
-        s.kerr, awp_wait_of(s));
+    k_vel_tma<TM, CW, S, 2><<<grid, dim3(32, CW + 1), smem, stream>>>(
+        st->vm, s.g, comp_set3(s), s.ncomp, s.staged_qslow, (const TM *)s.md.m[AM_D1], s.md.sc.inv[AM_D1], s.cx, s.cy,
+        s.cz, s.dth, w, s.kerr, awp_wait_of(s));
     return cudaGetLastError();
 }
+
+/* dynamic shared memory of a ring: alignment slack, slots, full + empty barriers */
+static size_t ring_bytes(int slots, int slot_floats) { return 128 + (size_t)slots * slot_floats * 4 + 2 * 8 * slots; }
 
 template <class TR, int UNR, int RPT>
 static cudaError_t launch_str_rpt(const AwpStaged *st, const AwpStepArgs &s, cudaStream_t stream)
@@ -1231,15 +900,6 @@ static cudaError_t launch_str_rpt(const AwpStaged *st, const AwpStepArgs &s, cud
     const size_t smem = ring_bytes(2 + STR_D, STR_SLOT);
     const AwpWork w = staged_work(s.g, s.kchunk_staged, s.ncomp);
     int grid = 0;
-    if (s.staged_generic && UNR == 2 && RPT == 1) {     /* generic ring loads (ring_base_t) */
-        cudaError_t e = staged_grid(k_str_tma<TR, 2, 1, true>, smem, w.nitems, &grid, s.sm_limit, 32 * (ST_Y + 1));
-        if (e != cudaSuccess) return e;
-        k_str_tma<TR, 2, 1, true><<<grid, dim3(32, ST_Y + 1), smem, stream>>>(st->sm, s.g, comp_set3(s), s.ncomp,
-                                                                            s.staged_qslow, s.cx, s.cy, s.cz, s.tau,
-                                                                            s.dth, s.dt, s.dh1, w, s.nve, s.kerr,
-                                                                            awp_wait_of(s));
-        return cudaGetLastError();
-    }
     cudaError_t e = staged_grid(k_str_tma<TR, UNR, RPT>, smem, w.nitems, &grid, s.sm_limit, 32 * (CW + 1));
     if (e != cudaSuccess) return e;
     k_str_tma<TR, UNR, RPT><<<grid, dim3(32, CW + 1), smem, stream>>>(st->sm, s.g, comp_set3(s), s.ncomp,
@@ -1284,37 +944,10 @@ static cudaError_t launch_str_tr(const AwpStaged *st, const AwpStepArgs &s, cuda
     return s.unroll == 1 ? launch_str_rpt<TR, 1, 1>(st, s, stream) : launch_str_rpt<TR, 2, 1>(st, s, stream);
 }
 
-template <int NCB, int CS>
-static cudaError_t launch_vel_b(const AwpStaged *st, const AwpStepArgs &s, cudaStream_t stream)
-{
-    const size_t smem = 128 + (size_t)(VB_MS * ST_MP + CS * VB_CSLOT) * 4 + 2 * 8 * (VB_MS + CS);
-    const AwpWork w = staged_work(s.g, s.kchunk_staged, 1);
-    int grid = 0;
-    cudaError_t e = staged_grid(k_vel_tmab<NCB, CS>, smem, w.nitems, &grid, s.sm_limit);
-    if (e != cudaSuccess) return e;
-    k_vel_tmab<NCB, CS><<<grid, dim3(32, ST_CW + 1), smem, stream>>>(
-        st->vm, s.g, comp_set3(s), (const float *)s.md.m[AM_D1], s.cx, s.cy, s.cz, s.dth, w, s.kerr, awp_wait_of(s));
-    return cudaGetLastError();
-}
-
-/* eight sub-slots (two blocks per SM): 1.20 ms per launch on the 400 x 400 x
- * 200 three-component grid against 1.28 with six, and 1.05 for one component
- * per item, which stays the default */
-template <int NCB>
-static cudaError_t launch_vel_bn(const AwpStaged *st, const AwpStepArgs &s, cudaStream_t stream)
-{
-    return launch_vel_b<NCB, 8>(st, s, stream);
-}
-
-/* level loops unrolled twice unless asked otherwise: the column queues then
- * rotate by register renaming instead of moves that wait for loads in flight */
 cudaError_t AWP_STAGED_ENTRY(awp_launch_vel_staged)(const AwpStaged *st, const AwpStepArgs &s, cudaStream_t stream)
 {
     if (!st || s.md.type != AWP_STORE_F32) return cudaErrorInvalidValue;
-    if ((s.staged_batch & 2) && s.ncomp == 3) return launch_vel_bn<3>(st, s, stream);
-    if ((s.staged_batch & 2) && s.ncomp == 2) return launch_vel_bn<2>(st, s, stream);
-    if (s.staged_rpt_vel == 2) return launch_vel_u<-1>(st, s, stream);
-    return s.unroll == 1 ? launch_vel_u<1>(st, s, stream) : launch_vel_u<2>(st, s, stream);
+    return launch_vel<float>(st, s, stream);
 }
 
 cudaError_t AWP_STAGED_ENTRY(awp_launch_str_staged)(const AwpStaged *st, const AwpStepArgs &s, cudaStream_t stream)

@@ -326,15 +326,16 @@ typedef struct {
     int staged_qslow;        /* staged sweeps: 1 = one component over all tiles first  */
     int staged_rpt;          /* staged stress sweep, one component per item: tile rows
                                 per thread (1, 2)                                      */
-    int staged_rpt_vel;      /* staged velocity sweep: tile rows per thread (1, 2)     */
+    int staged_rpt_vel;      /* accepted (1, 2) without effect: the staged velocity sweep
+                                has one form, two cells per thread                     */
     int unroll;              /* z-loop unroll of the sweeps (1, 2)                     */
     int ty;                  /* two-sweep / fused steppers: block rows (4, 8, 16)      */
     int kchunk;              /* fused stepper: z levels per work item (8..nz)          */
     int kchunk_sweep;        /* two-sweep stepper: z levels per work item (8..nz)      */
     int staged_batch;        /* staged sweeps with all components of a tile in one work
                                 item, sharing media tiles and cell coefficients:
-                                bit 0 the stress sweep, bit 1 the velocity sweep
-                                (default 1 up to 32 GiB of solver state, else 0) */
+                                bit 0 the stress sweep (default 1 up to 32 GiB of
+                                solver state, else 0); bit 1 accepted without effect */
     int sm_limit;            /* persistent grids sized for this many SMs (0 = every
                                 SM of the device): solves that share a GPU each take
                                 their share instead of time-slicing the whole device */
