@@ -650,7 +650,8 @@ k_str_tmab(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<
                 const int cm = (ty + r * CW + 1) * ST_W + tx + 4;
                 const int it = ipar | itxy[r];
                 const TMed M{mring + (mk % STB_MS) * STB_MSLOT + cm, mring + (mm % STB_MS) * STB_MSLOT + cm};
-                kc[r] = str_coef_t(M, nve, tau[it], tau[8 + it]);
+                if (live[r])          /* lanes outside the grid hold zero media: their divisions would be slow */
+                    kc[r] = str_coef_t(M, nve, tau[it], tau[8 + it]);
             }
             __syncwarp();
             if (tx == 0) mb_arrive(&mempty[mm % STB_MS]);
