@@ -120,7 +120,8 @@ struct AwpPostArgs {
     float dt;
     const void *mu;     /* typed compliance 1/mu (kinematic)     */
     float mu_inv;
-    float *kin[3];      /* [nsrc][6] per-step stress increments  */
+    const int *kin[3];  /* subfaults by cell: starts [nkin + 1], then the subfaults */
+    int nkin[3];        /* cells that hold subfaults             */
 };
 
 struct AwpSgtArgs {

@@ -23,6 +23,7 @@
 #include <new>
 #include <unordered_map>
 #include <utility>
+#include <algorithm>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -92,7 +93,8 @@ struct awp_solver {
     int kchunk;                      /* z levels per fused work item        */
     int kchunk_sweep;                /* z levels per two-sweep work item    */
     int staged_on;                   /* TMA-staged velocity/stress sweeps   */
-    float *kin[AWP_MAX_COMP];        /* kinematic subfault increments       */
+    int *kin[AWP_MAX_COMP];          /* kinematic subfaults by cell (k_kin) */
+    int nkin[AWP_MAX_COMP];
     size_t stagger;                  /* base-address offset step of the field arrays */
     int nstag;
     struct { void *user, *raw; } stag[AWP_MAX_FIELDS];   /* field arrays: pointer in use, block */
@@ -1133,11 +1135,29 @@ extern "C" awp_status awp_set_source(awp_solver *s, int comp, int nsrc, const in
     }
     awp_status st = dalloc(s, (void **)&s->src_ijk[comp], sizeof(int) * 3 * (size_t)nsrc);
     if (st == AWP_OK) st = dalloc(s, (void **)&s->src_stf[comp], sizeof(float) * 6 * (size_t)nsrc * (size_t)(p->nst > 0 ? p->nst : 1));
-    if (st == AWP_OK && p->kinematic) st = dalloc(s, (void **)&s->kin[comp], sizeof(float) * 6 * (size_t)nsrc);
+    std::vector<int> kin;             /* subfaults by cell: starts, then the subfaults cell by cell in their order */
+    if (p->kinematic) {
+        try {
+            std::vector<int> order(nsrc);
+            for (int m = 0; m < nsrc; m++) order[m] = m;
+            auto cell = [&](int m) { return s->g.idx(ijk[3 * m], ijk[3 * m + 1], ijk[3 * m + 2]); };
+            std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cell(a) < cell(b); });
+            for (int e = 0; e < nsrc; e++)
+                if (e == 0 || cell(order[e]) != cell(order[e - 1])) kin.push_back(e);
+            s->nkin[comp] = (int)kin.size();
+            kin.push_back(nsrc);
+            kin.insert(kin.end(), order.begin(), order.end());
+        } catch (const std::bad_alloc &) {
+            st = set_err(AWP_ERR_OOM, "host allocation failed");
+        }
+        if (st == AWP_OK) st = dalloc(s, (void **)&s->kin[comp], sizeof(int) * kin.size());
+    }
     if (st == AWP_OK) {
         cudaError_t e = cudaMemcpy(s->src_ijk[comp], ijk, sizeof(int) * 3 * (size_t)nsrc, cudaMemcpyHostToDevice);
         if (e == cudaSuccess && p->nst > 0)
             e = cudaMemcpy(s->src_stf[comp], stf, sizeof(float) * 6 * (size_t)nsrc * (size_t)p->nst, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && !kin.empty())
+            e = cudaMemcpy(s->kin[comp], kin.data(), sizeof(int) * kin.size(), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) st = set_err(AWP_ERR_CUDA, "source upload: %s", cudaGetErrorString(e));
     }
     free(ijk);
@@ -1244,6 +1264,7 @@ static void fill_args(awp_solver *s, int steps, AwpStepArgs &a, AwpPostArgs &pa,
         pa.src[q].ijk = s->src_ijk[q];
         pa.src[q].stf = s->src_stf[q];
         pa.kin[q] = s->kin[q];
+        pa.nkin[q] = s->kin[q] ? s->nkin[q] : 0;
         pa.comp[q] = s->comp[wr][q];
     }
 

@@ -1,0 +1,41 @@
+"""Kinematic sources that fill several thread blocks, against the FP32 oracle."""
+import numpy as np
+import pytest
+
+import awp_inputs as ai
+import awpsgt
+import oracle
+
+from test_gpu_parity import kinematic_rupture, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 128, 129, 400])
+def test_kinematic_subfaults_over_several_blocks(n):
+    """One thread per cell that holds subfaults: block edges, and cells shared
+    by many subfaults (every third one falls on one of four cells).  The
+    tolerance is the kinematic parity test's: the CUDA and C-library sines and
+    exponentials differ in the last bits."""
+    nx, ny, nz, nt, dt = 48, 40, 32, 40, 0.01
+    xyz = [(10 + k % 28, 12 + (k // 28) % 14, 6 + k % 9) for k in range(n)]
+    xyz = [(20 + (k // 3) % 4, 20, 12) if k % 3 == 2 else c for k, c in enumerate(xyz)]
+    tab = kinematic_rupture(n, dt=dt)
+    media = ai.layered_media(nx, ny, nz, 200.0, seed=3, pert_std=0.05, corr_len=1000.0)
+    pts = ai.sgt_points(nx, ny, 20, 50, seed=0)
+    kw = dict(nd=8, socalq=1, ntiskp_sgt=5, write_step=4, fl=0.01, fh=25.0, fp=0.5)
+    p = awpsgt.make_params(nx, ny, nz, 200.0, dt, nt, nst=2, igreen=(1,), kinematic=1, **kw)
+    with awpsgt.Solver(p) as s:
+        s.load_media(media)
+        s.set_source(0, xyz, tab)
+        s.set_points(pts)
+        s.run(nt)
+        g, gxx = s.sgt(0), s.field("xx")
+    o = oracle.Oracle(nx=nx, ny=ny, nz=nz, dh=200.0, dt=dt, nt=nt, nst=2, igreen=1, kinematic=1, precision="f32", **kw)
+    o.load_media(media)
+    o.set_source(xyz, tab)
+    o.set_points(pts)
+    o.run(nt)
+    assert np.abs(g).max() > 0
+    assert rel_l2(g, o.sgt()) <= 1e-5
+    assert rel_l2(gxx, o.field("xx")) <= 1e-5
