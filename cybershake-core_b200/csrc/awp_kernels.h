@@ -49,7 +49,7 @@ struct AwpStepArgs {
     int ty;                      /* thread-block rows (4, 8 or 16)          */
     int unroll;                  /* two-sweep z-loop unroll (1 or 2)        */
     const AwpStaged *staged;     /* non-NULL: TMA-staged velocity/stress    */
-    int kchunk_staged;           /* z levels per staged work item           */
+    int kchunk_staged;           /* z levels per staged work item (0: each sweep picks) */
     int staged_qslow;            /* staged items: one component at a time   */
     int staged_rpt;              /* staged stress sweep: tile rows per thread */
     int staged_batch;            /* bit 0: staged stress sweep with the components side by side in one item */

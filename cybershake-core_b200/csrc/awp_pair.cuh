@@ -119,7 +119,7 @@ k_vel_tma(const __grid_constant__ AwpStagedVelMaps maps, AwpGeom g, AwpCompSet<A
             int q, t;
             split_item(item, ncomp, w.nitems / ncomp, qslow, q, t);
             int bx, by, k0, k1;
-            work_item(g, w, t, bx, by, k0, k1);
+            staged_item(g, w, t, bx, by, k0, k1);
             const int j0 = by * ROWS + 1, xp = bx * PR_X + AWP_XO, x = xp - 4;
             for (int k = k0; k <= k1; ++k, ++use) {
                 ok = ring_acquire<S>(empty, use, &abort_s, wt.ns);
@@ -155,7 +155,7 @@ k_vel_tma(const __grid_constant__ AwpStagedVelMaps maps, AwpGeom g, AwpCompSet<A
         int q, t;
         split_item(item, ncomp, w.nitems / ncomp, qslow, q, t);
         int bx, by, k0, k1;
-        work_item(g, w, t, bx, by, k0, k1);
+        staged_item(g, w, t, bx, by, k0, k1);
         const int i = bx * PR_X + 1 + lx, j = by * ROWS + 1 + row;
         const int live = j <= g.ny ? max(0, min(2, g.nx - i + 1)) : 0;
         float *U = pick(cs, q, AF_U), *V = pick(cs, q, AF_V), *W = pick(cs, q, AF_W);

@@ -99,6 +99,7 @@ struct awp_solver {
     int nstag;
     struct { void *user, *raw; } stag[AWP_MAX_FIELDS];   /* field arrays: pointer in use, block */
     int kchunk_staged;               /* z levels per staged work item       */
+    int kchunk_auto;                 /* not set by anyone: each sweep picks its own (awp_staged.cu) */
     int staged_qslow;                /* staged items: component slowest     */
     int staged_rpt;                  /* staged stress sweep rows per thread */
     int staged_rpt_vel;              /* staged velocity sweep rows per thread */
@@ -702,9 +703,11 @@ extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
     s->kchunk = choose_kchunk(s->g, 1, s->ty);
     s->kchunk_sweep = choose_kchunk(s->g, 0, s->ty == 4 ? 4 : 8);
     {
-        /* z chunks of about 40 levels, split evenly: every chunk costs one
-         * prologue level, and a short last chunk leaves blocks idle */
+        /* z chunks: each sweep picks its own from the grid and its resident
+         * blocks unless told otherwise; what awp_get_tuning reports then is
+         * about 40 levels, split evenly */
         int kc = env_int("AWP_TUNE_KSTAGE", 0);
+        s->kchunk_auto = kc <= 0;
         if (kc <= 0) {
             const int nch = (s->g.nz + 39) / 40;
             kc = (s->g.nz + nch - 1) / nch;
@@ -1233,7 +1236,7 @@ static void fill_args(awp_solver *s, int steps, AwpStepArgs &a, AwpPostArgs &pa,
     a.ty = s->ty;
     a.unroll = s->unroll;
     a.staged = s->staged_on ? s->staged : NULL;
-    a.kchunk_staged = s->kchunk_staged;
+    a.kchunk_staged = s->kchunk_auto ? 0 : s->kchunk_staged;
     a.staged_qslow = s->staged_qslow;
     a.staged_rpt = s->staged_rpt;
     a.staged_batch = s->staged_batch;
@@ -2254,6 +2257,7 @@ extern "C" awp_status awp_set_tuning(awp_solver *s, const awp_tuning *t)
                        "0-3, sm_limit >= 0");
     CU(cudaSetDevice(s->p.device));
     CU(cudaStreamSynchronize(s->stream));   /* no captured step in flight when its graph goes */
+    if (s->kchunk_staged != t->kchunk_staged) s->kchunk_auto = 0;
     s->kchunk_staged = t->kchunk_staged;
     s->staged_qslow = t->staged_qslow;
     s->staged_rpt = t->staged_rpt;

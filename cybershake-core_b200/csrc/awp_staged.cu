@@ -147,6 +147,18 @@ __device__ __forceinline__ void tma_3d(void *dst, const CUtensorMap *map, uint64
  * j0 - 1 (media), level k */
 __device__ __forceinline__ int tile_x(int i0) { return i0 + AWP_XO - 1 - 4; }
 
+/* tile and levels of a work item: nzc chunks that differ by a level at most */
+__device__ __forceinline__ void staged_item(const AwpGeom &g, const AwpWork &w, int item, int &bx, int &by, int &k0,
+                                            int &k1)
+{
+    bx = item % w.ntx;
+    const int t = item / w.ntx;
+    by = t % w.nty;
+    const int bz = t / w.nty;
+    k0 = bz * g.nz / w.nzc + 1;
+    k1 = (bz + 1) * g.nz / w.nzc;
+}
+
 /* component q and tile item t of work item `item`: the components of one
  * tile side by side (qslow = 0; their common media tiles come from L2) or one
  * component over all tiles at a time (qslow = 1; fewer arrays streamed at once) */
@@ -381,7 +393,7 @@ k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<A
             int q, t;
             split_item(item, ncomp, w.nitems / ncomp, qslow, q, t);
             int bx, by, k0, k1;
-            work_item(g, w, t, bx, by, k0, k1);
+            staged_item(g, w, t, bx, by, k0, k1);
             for (int k = k0 - 1; k <= k1; ++k, ++use) {
                 ok = ring_acquire<S>(empty, use, &abort_s, wt.ns);
                 if (!ok) break;
@@ -403,7 +415,7 @@ k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<A
         int q, t;
         split_item(item, ncomp, w.nitems / ncomp, qslow, q, t);
         int bx, by, k0, k1;
-        work_item(g, w, t, bx, by, k0, k1);
+        staged_item(g, w, t, bx, by, k0, k1);
         const int i = bx * ST_X + 1 + tx;
         const int np = k1 - k0 + 2;   /* levels k0-1 .. k1 */
         const float *U = tab[q].f[AF_U], *V = tab[q].f[AF_V], *W = tab[q].f[AF_W];
@@ -553,7 +565,7 @@ k_str_tmab(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<
         const int nmed = nve == 1 ? 4 : 2;
         for (int item = blockIdx.x; ok && item < w.nitems; item += gridDim.x) {
             int bx, by, k0, k1;
-            work_item(g, w, item, bx, by, k0, k1);
+            staged_item(g, w, item, bx, by, k0, k1);
             const int i0 = bx * ST_X + 1, j0 = by * ST_Y + 1;
             const int x = tile_x(i0), xp = i0 + AWP_XO - 1;
             for (int k = k0 - 1; ok && k <= k1; ++k) {
@@ -598,7 +610,7 @@ k_str_tmab(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<
     uint32_t um0 = 0, uc = 0;         /* media use of the item's level k0 - 1; next component use */
     for (int item = blockIdx.x; item < w.nitems; item += gridDim.x) {
         int bx, by, k0, k1;
-        work_item(g, w, item, bx, by, k0, k1);
+        staged_item(g, w, item, bx, by, k0, k1);
         const int i = bx * ST_X + 1 + tx;
         const int c0 = g.idx(i, by * ST_Y + 1 + ty, k0);
         /* per row and component: column queues u, v at k+1, k+2 and w at k+1,
@@ -831,30 +843,73 @@ static AwpWait awp_wait_of(const AwpStepArgs &s)
     return w;
 }
 
-static AwpWork staged_work(const AwpGeom &g, int kchunk, int ncomp)
+/* SMs a launch may use and resident blocks of the kernel on one of them */
+struct StagedSlots {
+    int nsm, per;
+};
+
+template <class K>
+static cudaError_t staged_slots(K kernel, size_t smem, int sm_limit, int threads, StagedSlots *o)
+{
+    int dev = 0;
+    o->nsm = 148;
+    o->per = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&o->nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (sm_limit > 0 && sm_limit < o->nsm) o->nsm = sm_limit;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o->per, kernel, threads, smem);
+    if (e != cudaSuccess) return e;
+    return o->per < 1 ? cudaErrorInvalidConfiguration : cudaSuccess;
+}
+
+/* z chunks of a sweep over `tiles` column tiles.  An item costs
+ * its levels plus about `extra` for its prologue (the planes below its first
+ * level, column values from global memory, the first copies).  Items run in
+ * rounds of nsm * per; a full SM works through them at one level per unit of
+ * time and block, and an SM with fewer blocks is bound by the latency of a
+ * level, about 0.65 * per units.  The split with the least time by that count
+ * is taken: on a grid that fills the device it keeps the last round full, on
+ * a small one it spreads the columns over all SMs (100x100x50, one component:
+ * chunks of 7 levels instead of 25).  At least five levels: the prologue must
+ * not outweigh them, and the top chunk's threads mirror the levels nz-2 .. nz
+ * themselves.  Steps, fixed 25 .. 40 levels before -> this rule: 100x100x50 one
+ * component 0.052 -> 0.037 ms, 160x160x80 0.114 -> 0.084, 120x110x60 two
+ * components 0.114 -> 0.072, 400x400x200 three 3.18 -> 3.11. */
+static int pick_chunks(int nz, int tiles, const StagedSlots &sl, double extra)
+{
+    const int slots = sl.nsm * sl.per, kmin = nz < 5 ? nz : 5;
+    int best = 1;
+    double best_t = 1e30;
+    for (int n = 1; n * kmin <= nz; ++n) {
+        const long long items = (long long)tiles * n;
+        const int rem = (int)(items % slots), on_sm = (rem + sl.nsm - 1) / sl.nsm;
+        const double tail = rem ? (on_sm > 0.65 * sl.per ? on_sm : 0.65 * sl.per) : 0.0;
+        const double t = ((double)nz / n + extra) * ((double)(items / slots) * sl.per + tail);
+        if (t < best_t) {
+            best_t = t;
+            best = n;
+        }
+    }
+    return best;
+}
+
+/* work items of a sweep over 32 x rows tiles; kchunk: most levels of an item, 0: pick_chunks */
+static AwpWork staged_work(const AwpGeom &g, int rows, int kchunk, int ncomp, const StagedSlots &sl, double extra)
 {
     AwpWork w;
     w.ntx = (g.nx + ST_X - 1) / ST_X;
-    w.nty = (g.ny + ST_Y - 1) / ST_Y;
+    w.nty = (g.ny + rows - 1) / rows;
     w.kchunk = kchunk;
-    w.nzc = (g.nz + kchunk - 1) / kchunk;
+    w.nzc = kchunk > 0 ? (g.nz + kchunk - 1) / kchunk : pick_chunks(g.nz, w.ntx * w.nty * ncomp, sl, extra);
     w.nitems = w.ntx * w.nty * w.nzc * ncomp;
     return w;
 }
 
-template <class K>
-static cudaError_t staged_grid(K kernel, size_t smem, int nitems, int *grid, int sm_limit, int threads = ST_THREADS)
+static int staged_grid(const StagedSlots &sl, const AwpWork &w)
 {
-    int dev = 0, nsm = 148, per = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (sm_limit > 0 && sm_limit < nsm) nsm = sm_limit;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
-    if (e != cudaSuccess) return e;
-    if (per < 1) return cudaErrorInvalidConfiguration;
-    *grid = nsm * per < nitems ? nsm * per : nitems;
-    return cudaSuccess;
+    const int n = sl.nsm * sl.per;
+    return n < w.nitems ? n : w.nitems;
 }
 
 static AwpCompSet<AWP_MAX_COMP> comp_set3(const AwpStepArgs &s)
@@ -865,27 +920,16 @@ static AwpCompSet<AWP_MAX_COMP> comp_set3(const AwpStepArgs &s)
     return cs;
 }
 
-static AwpWork pair_work(const AwpGeom &g, int rows, int kchunk, int ncomp)
-{
-    AwpWork w;
-    w.ntx = (g.nx + PR_X - 1) / PR_X;
-    w.nty = (g.ny + rows - 1) / rows;
-    w.kchunk = kchunk;
-    w.nzc = (g.nz + kchunk - 1) / kchunk;
-    w.nitems = w.ntx * w.nty * w.nzc * ncomp;
-    return w;
-}
-
 template <class TM>
 static cudaError_t launch_vel(const AwpStaged *st, const AwpStepArgs &s, cudaStream_t stream)
 {
     constexpr int CW = PR_VEL_CW, S = 3;
     const size_t smem = PairVelL<TM, CW>::smem(S);
-    const AwpWork w = pair_work(s.g, 2 * CW, s.kchunk_staged, s.ncomp);
-    int grid = 0;
-    cudaError_t e = staged_grid(k_vel_tma<TM, CW, S, 2>, smem, w.nitems, &grid, s.sm_limit, 32 * (CW + 1));
+    StagedSlots sl;
+    cudaError_t e = staged_slots(k_vel_tma<TM, CW, S, 2>, smem, s.sm_limit, 32 * (CW + 1), &sl);
     if (e != cudaSuccess) return e;
-    k_vel_tma<TM, CW, S, 2><<<grid, dim3(32, CW + 1), smem, stream>>>(
+    const AwpWork w = staged_work(s.g, 2 * CW, s.kchunk_staged, s.ncomp, sl, 1.0);
+    k_vel_tma<TM, CW, S, 2><<<staged_grid(sl, w), dim3(32, CW + 1), smem, stream>>>(
         st->vm, s.g, comp_set3(s), s.ncomp, s.staged_qslow, (const TM *)s.md.m[AM_D1], s.md.sc.inv[AM_D1], s.cx, s.cy,
         s.cz, s.dth, w, s.kerr, awp_wait_of(s));
     return cudaGetLastError();
@@ -899,11 +943,11 @@ static cudaError_t launch_str_rpt(const AwpStaged *st, const AwpStepArgs &s, cud
 {
     constexpr int CW = ST_Y / RPT;
     const size_t smem = ring_bytes(2 + STR_D, STR_SLOT);
-    const AwpWork w = staged_work(s.g, s.kchunk_staged, s.ncomp);
-    int grid = 0;
-    cudaError_t e = staged_grid(k_str_tma<TR, UNR, RPT>, smem, w.nitems, &grid, s.sm_limit, 32 * (CW + 1));
+    StagedSlots sl;
+    cudaError_t e = staged_slots(k_str_tma<TR, UNR, RPT>, smem, s.sm_limit, 32 * (CW + 1), &sl);
     if (e != cudaSuccess) return e;
-    k_str_tma<TR, UNR, RPT><<<grid, dim3(32, CW + 1), smem, stream>>>(st->sm, s.g, comp_set3(s), s.ncomp,
+    const AwpWork w = staged_work(s.g, ST_Y, s.kchunk_staged, s.ncomp, sl, 1.5);
+    k_str_tma<TR, UNR, RPT><<<staged_grid(sl, w), dim3(32, CW + 1), smem, stream>>>(st->sm, s.g, comp_set3(s), s.ncomp,
                                                                        s.staged_qslow, s.cx, s.cy, s.cz, s.tau,
                                                                        s.dth, s.dt, s.dh1, w, s.nve, s.kerr, awp_wait_of(s));
     return cudaGetLastError();
@@ -915,11 +959,11 @@ static cudaError_t launch_str_bc(const AwpStaged *st, const AwpStepArgs &s, cuda
 {
     constexpr int CW = ST_Y / RPT;
     const size_t smem = 128 + (size_t)(STB_MS * STB_MSLOT + CS * STB_CSLOT) * 4 + 2 * 8 * (STB_MS + CS);
-    const AwpWork w = staged_work(s.g, s.kchunk_staged, 1);
-    int grid = 0;
-    cudaError_t e = staged_grid(k_str_tmab<TR, NCB, CS, RPT>, smem, w.nitems, &grid, s.sm_limit, 32 * (CW + 1));
+    StagedSlots sl;
+    cudaError_t e = staged_slots(k_str_tmab<TR, NCB, CS, RPT>, smem, s.sm_limit, 32 * (CW + 1), &sl);
     if (e != cudaSuccess) return e;
-    k_str_tmab<TR, NCB, CS, RPT><<<grid, dim3(32, CW + 1), smem, stream>>>(
+    const AwpWork w = staged_work(s.g, ST_Y, s.kchunk_staged, 1, sl, 1.0);
+    k_str_tmab<TR, NCB, CS, RPT><<<staged_grid(sl, w), dim3(32, CW + 1), smem, stream>>>(
         st->sm, s.g, comp_set3(s), s.cx, s.cy, s.cz, s.tau, s.dth, s.dt, s.dh1, w, s.nve, s.kerr, awp_wait_of(s));
     return cudaGetLastError();
 }

@@ -1,4 +1,5 @@
-"""Kinematic sources that fill several thread blocks, against the FP32 oracle."""
+"""The staged sweeps at the edges of their tiles and z chunks, and kinematic
+sources that fill several thread blocks, against the FP32 oracle."""
 import numpy as np
 import pytest
 
@@ -6,9 +7,25 @@ import awp_inputs as ai
 import awpsgt
 import oracle
 
-from test_gpu_parity import kinematic_rupture, rel_l2
+from test_gpu_parity import Case, assert_same_state, kinematic_rupture, rel_l2
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nx,ny,nz,igreen", [
+    (8, 8, 8, (1,)), (31, 15, 9, (1,)), (32, 16, 10, (1, 2)), (33, 17, 11, (1, 2, 3)), (34, 31, 12, (3,)),
+    (63, 33, 8, (1, 2)), (65, 18, 21, (2,)), (95, 47, 14, (1, 2, 3)),
+])
+def test_tile_and_chunk_edges_are_bit_exact(nx, ny, nz, igreen):
+    """Pairs of cells cut by the grid's edge, partial tiles in x and y, chunks
+    of the automatic rule down to five levels: every field, CHKJ and the SGT
+    image bit for bit."""
+    c = Case(nx=nx, ny=ny, nz=nz, nt=12, igreen=igreen, nd=3, npts=20,
+             srcs=[[(nx // 2 + 1, ny // 2 + 1, nz // 2)]] * len(igreen), ntiskp=3, write_step=2)
+    s = c.gpu(kernel="staged")
+    for q in range(len(igreen)):
+        assert_same_state(s, c.oracle(q), q)
+    s.close()
 
 
 @pytest.mark.parametrize("n", [1, 128, 129, 400])
