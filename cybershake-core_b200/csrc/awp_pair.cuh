@@ -28,16 +28,22 @@
 
 __host__ __device__ constexpr int pr_pad(int n) { return (n + 31) / 32 * 32; }   /* 128-byte tiles */
 
-/* media tile row of storage type TM: elements from cell i0 on (the averages
- * reach one cell up in x), a multiple of 16 bytes */
-template <class TM> struct MedRow { static constexpr int W = 40; };
-template <> struct MedRow<float> { static constexpr int W = 36; };
-
 /* three consecutive media values */
 __device__ __forceinline__ void med3(const float *p, float, float m[3])
 {
     const float2 a = *(const float2 *)p, b = *(const float2 *)(p + 2);
     m[0] = a.x; m[1] = a.y; m[2] = b.x;
+}
+
+__device__ __forceinline__ void med3(const __nv_bfloat16 *p, float, float m[3])
+{
+    const __nv_bfloat162 a = *(const __nv_bfloat162 *)p;
+    m[0] = __low2float(a); m[1] = __high2float(a); m[2] = __bfloat162float(p[2]);
+}
+__device__ __forceinline__ void med3(const __half *p, float inv, float m[3])
+{
+    const __half2 a = *(const __half2 *)p;
+    m[0] = __low2float(a) * inv; m[1] = __high2float(a) * inv; m[2] = __half2float(p[2]) * inv;
 }
 
 __device__ __forceinline__ float2 ld2(const float *p) { return *(const float2 *)p; }

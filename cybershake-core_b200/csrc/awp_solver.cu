@@ -627,7 +627,7 @@ extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
     for (int m = 0; m < AM_N; m++) { s->mdt.sc.scale[m] = 1.0f; s->mdt.sc.inv[m] = 1.0f; }
     if (s->store != AWP_STORE_F32)
         for (int m = 0; m < AM_N; m++) {
-            TRY(dalloc(s, &s->mdt.m[m], (size_t)s->g.vol * 2));
+            TRY(dalloc_field(s, &s->mdt.m[m], (size_t)s->g.vol * 2, 2));
             TRYCU(cudaMemsetAsync(s->mdt.m[m], 0, (size_t)s->g.vol * 2, s->stream));
         }
     /* sponge factors (cerjan.f:19-242): separable, both lateral faces and
@@ -695,7 +695,7 @@ extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
     s->ty = env_int("AWP_TUNE_TY", 8);
     if (s->ty != 4 && s->ty != 16) s->ty = 8;
     s->staged_on = p->kernel == AWP_KERNEL_STAGED || p->kernel == AWP_KERNEL_STAGED_FMA ||
-                   (p->kernel == AWP_KERNEL_AUTO && s->store == AWP_STORE_F32);
+                   p->kernel == AWP_KERNEL_AUTO;
     s->fma = p->kernel == AWP_KERNEL_STAGED_FMA;
     /* z-loop unroll: 1 or 2 (default 1 for the two-sweep kernels, 2 for the staged ones) */
     s->unroll = env_int("AWP_TUNE_UNROLL", 0);
