@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Benchmark of the B200 AWP-ODC-SGT stepper (Gcell-updates/s), default
-TMA-staged two-sweep kernels (k_vel_tma, k_fsvel, k_str_tma).
+TMA-staged two-sweep kernels (k_vel_tma, k_str_tma / k_str_tmab).
 
 Workload: the batched fx+fy+fz SGT solve on a 400x400x200 grid (h = 100 m,
 dt = 0.005 s, 4000 source steps, 5000 SGT points every 10 steps), seeded
@@ -723,7 +723,8 @@ def main():
                 "step_frac": (step_bytes * value * 1e9 / (cells * ncomp * world)) / 1e9 / peak,
                 "bytes_per_cell_update": bpcu}
 
-    launches_per_ts = (2 if "k_fused" in prof else 4) + 2 * boundary(w)   # stepper kernel(s) + k_post (+ PML)
+    # stepper kernels and k_post (the staged stress sweep includes k_fsvel's work, and k_post's without the PML)
+    launches_per_ts = 2 if "k_fused" in prof else (4 if "k_vel_tma" not in prof else 2 + boundary(w)) + 3 * boundary(w)
     gpu_launches = args.steps * (per_step_ts * launches_per_ts + 1)
 
     line = {

@@ -31,6 +31,7 @@
 #include "awp_internal.h"
 #include "awp_kernels.h"
 #include "awp_stencil.cuh"
+#include "awp_post.cuh"
 
 /* ------------------------------------------------------------------ */
 /* media                                                               */
@@ -505,113 +506,8 @@ k_fused(AwpGeom g, MediaT<TM> md, AwpCompSet<NC> old, AwpCompSet<NC> nw, const f
 /* per-step serial work: source insertion, fstr redo, CHKJ probe       */
 /* ------------------------------------------------------------------ */
 
-__device__ void fstr_column(const AwpGeom &g, AwpComp &cp, int i, int j)
-{
-    const int nz = g.nz, sz = g.plane;
-    const int c = g.idx(i, j, nz);
-    float *zz = cp.f[AF_ZZ], *xz = cp.f[AF_XZ], *yz = cp.f[AF_YZ];
-    zz[c + sz] = -zz[c];
-    zz[c + 2 * sz] = -zz[c - sz];
-    xz[c + sz] = -xz[c - sz];
-    xz[c + 2 * sz] = -xz[c - 2 * sz];
-    yz[c + sz] = -yz[c - sz];
-    yz[c + 2 * sz] = -yz[c - 2 * sz];
-    xz[c] = 0.0f;
-    yz[c] = 0.0f;
-}
-
-__device__ __forceinline__ float d1_at(const AwpPostArgs &a, int c)
-{
-    switch (a.media_type) {
-    case 1: return __bfloat162float(((const __nv_bfloat16 *)a.d1)[c]);
-    case 2: return __half2float(((const __half *)a.d1)[c]) * a.d1_inv;
-    default: return ((const float *)a.d1)[c];
-    }
-}
-
-/* One block; thread q handles component q and walks its sources in order,
- * as the Fortran loop over j=1,npsrc does.
- * initial != 0: addsrc(1) before the time loop (pmcl3d.f:966-988).
- * otherwise: step n = *step + 1 just finished its stress update:
- *   addsrc(n+1) [and fstr again where a moment source sits in the top three
- *   layers, since pmcl3d.f:1383-1384 inserts before fstr], CHKJ sample,
- *   then *step = n. */
-__global__ void k_post(AwpPostArgs a, int initial)
-{
-    const int q = threadIdx.x;
-    const int n = initial ? 0 : (*a.step + 1);
-    const int sample = initial ? 1 : n + 1;
-    if (q < a.ncomp && sample <= a.nst && !a.kinematic) {
-        const AwpSrcDev &s = a.src[q];
-        AwpComp &cp = a.comp[q];
-        const AwpGeom &g = a.g;
-        const int nz = g.nz, sz = g.plane;
-        for (int m = 0; m < s.nsrc; ++m) {
-            const int i = s.ijk[3 * m], j = s.ijk[3 * m + 1], k = s.ijk[3 * m + 2];
-            const float *t = s.stf + ((int64_t)m * a.nst + (sample - 1)) * 6;
-            const float axx = t[0], ayy = t[1], azz = t[2], axz = t[3], ayz = t[4], axy = t[5];
-            const int c = g.idx(i, j, k);
-            const int ct = g.idx(i, j, nz);
-            switch (s.igreen) {
-            case -1:
-                cp.f[AF_XX][c] = cp.f[AF_XX][c] - a.vtst * axx;
-                cp.f[AF_YY][c] = cp.f[AF_YY][c] - a.vtst * ayy;
-                cp.f[AF_ZZ][c] = cp.f[AF_ZZ][c] - a.vtst * azz;
-                cp.f[AF_XZ][c] = cp.f[AF_XZ][c] - a.vtst * axz;
-                cp.f[AF_YZ][c] = cp.f[AF_YZ][c] - a.vtst * ayz;
-                cp.f[AF_XY][c] = cp.f[AF_XY][c] - a.vtst * axy;
-                break;
-            case 1:
-                cp.f[AF_U][c] = cp.f[AF_U][c] + axx * a.vtst / d1_at(a, c);
-                break;
-            case 2:
-                cp.f[AF_V][c] = cp.f[AF_V][c] + ayy * a.vtst / d1_at(a, c);
-                break;
-            case 3:
-                cp.f[AF_W][c] = cp.f[AF_W][c] + azz * a.vtst / d1_at(a, c);
-                break;
-            case -2:
-                cp.f[AF_U][c] = cp.f[AF_U][c] + axx * a.vtst / d1_at(a, c);
-                cp.f[AF_V][c] = cp.f[AF_V][c] + ayy * a.vtst / d1_at(a, c);
-                cp.f[AF_W][c] = cp.f[AF_W][c] + azz * a.vtst / d1_at(a, c);
-                break;
-            case 4: {
-                float *F = cp.f[AF_XZ];
-                F[ct] = axx * a.vtst1;
-                F[ct + sz] = 2.0f * axx * a.vtst1 - F[ct - sz];
-                F[ct + 2 * sz] = 2.0f * axx * a.vtst1 - F[ct - 2 * sz];
-            } break;
-            case 5: {
-                float *F = cp.f[AF_YZ];
-                F[ct] = ayy * a.vtst1;
-                F[ct + sz] = 2.0f * ayy * a.vtst1 - F[ct - sz];
-                F[ct + 2 * sz] = 2.0f * ayy * a.vtst1 - F[ct - 2 * sz];
-            } break;
-            case 6: {
-                float *F = cp.f[AF_ZZ];
-                F[ct + sz] = 2.0f * azz * a.vtst1 - F[ct];
-                F[ct + 2 * sz] = 2.0f * azz * a.vtst1 - F[ct - sz];
-            } break;
-            default:
-                break;
-            }
-        }
-        if (!initial && s.igreen == -1) {
-            for (int m = 0; m < s.nsrc; ++m)
-                if (s.ijk[3 * m + 2] >= nz - 2) fstr_column(g, cp, s.ijk[3 * m], s.ijk[3 * m + 1]);
-        }
-    }
-    if (initial) return;
-    __syncthreads();
-    if (q < a.ncomp && a.probe > 0 && n >= 1 && n <= a.nt) {
-        const int c = a.g.idx(a.probe, a.probe, a.probe);
-        a.chkj[q][3 * (n - 1)] = a.comp[q].f[AF_U][c];
-        a.chkj[q][3 * (n - 1) + 1] = a.comp[q].f[AF_V][c];
-        a.chkj[q][3 * (n - 1) + 2] = a.comp[q].f[AF_W][c];
-    }
-    __syncthreads();
-    if (q == 0) *a.step = n;
-}
+/* one warp (step_post.cuh) */
+__global__ void k_post(AwpPostArgs a, int initial) { step_post(a, initial); }
 
 /* SGT gather, pmcl3d.f:1537-1557.  Sample s (0-based) of every point goes
  * straight to its place in the raw file image, [pt][6][nt_file]. */
@@ -921,6 +817,7 @@ cudaError_t awp_launch_step(const AwpStepArgs &s, cudaStream_t st)
 {
     if (s.fused) return awp_launch_part(s, AWP_PART_FUSED, st);
     for (int part = 0; part < 3; ++part) {
+        if (part == AWP_PART_FSVEL && s.staged) continue;      /* part of the staged stress sweep */
         cudaError_t e = awp_launch_part(s, part, st);
         /* NPC = 1: the PML zones recomputed after the velocity sweep (before
          * the free-surface velocity) and after the stress sweep */

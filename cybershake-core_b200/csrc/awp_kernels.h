@@ -58,6 +58,8 @@ struct AwpStepArgs {
     int fma;                     /* staged sweeps compiled with multiply-add contraction */
     const AwpPmlArgs *pml;       /* NPC = 1: the PML zones after each sweep (NULL: Cerjan) */
     unsigned long long wait_ns;  /* bound of one barrier wait of the staged sweeps */
+    const AwpPostArgs *post;     /* staged: the stress sweep also does the step's serial work (NULL: k_post) */
+    int *post_done;              /* its warp count, zero between launches    */
     int withhold;                /* test injection, -1 = off: block 0's producer of the
                                     staged stress sweep issues no copies for ring use
                                     `withhold`, so its consumers' wait runs out */

@@ -124,7 +124,8 @@ struct awp_solver {
     /* stability monitor */
     double *en_partial;              /* scratch: AWP_EN_GRID * ncomp       */
     double *en_out;                  /* last energy per component          */
-    int *flag;                       /* set by the monitor on NaN/Inf      */
+    int *flag;                       /* [0] set by the monitor on NaN/Inf, [1] AWP_KERR_*,
+                                        [2] finished warps of a stress sweep (AwpStepArgs::post_done) */
     int next_check;
     int pending;                     /* asynchronous steps not yet synced  */
     int pending_steps;
@@ -680,9 +681,9 @@ extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
     TRY(dalloc(s, (void **)&s->rng, 2 * AM_N * sizeof(unsigned)));
     TRY(dalloc(s, (void **)&s->en_partial, sizeof(double) * AWP_EN_GRID * AWP_MAX_COMP));
     TRY(dalloc(s, (void **)&s->en_out, sizeof(double) * AWP_MAX_COMP));
-    TRY(dalloc(s, (void **)&s->flag, 2 * sizeof(int)));   /* [0] monitor, [1] AWP_KERR_* */
+    TRY(dalloc(s, (void **)&s->flag, 3 * sizeof(int)));
     TRYCU(cudaMemsetAsync(s->en_out, 0, sizeof(double) * AWP_MAX_COMP, s->stream));
-    TRYCU(cudaMemsetAsync(s->flag, 0, 2 * sizeof(int), s->stream));
+    TRYCU(cudaMemsetAsync(s->flag, 0, 3 * sizeof(int), s->stream));
     s->next_check = p->monitor_every > 0 ? p->monitor_every : 0;
     for (int q = 0; q < p->ncomp; q++) {
         TRY(dalloc(s, (void **)&s->chkj[q], sizeof(float) * 3 * (size_t)p->nt));
@@ -1287,8 +1288,11 @@ static cudaError_t enqueue_one(awp_solver *s, int steps)
 {
     AwpStepArgs a; AwpPostArgs pa; AwpSgtArgs sa;
     fill_args(s, steps, a, pa, sa);
+    /* the staged stress sweep ends with the serial work itself, unless other
+     * kernels still change the stresses after it */
+    if (a.staged && !a.pml && !s->p.kinematic) { a.post = &pa; a.post_done = s->flag + 2; }
     cudaError_t e = awp_launch_step(a, s->stream);
-    if (e == cudaSuccess) e = awp_launch_post(pa, 0, s->stream);
+    if (e == cudaSuccess && !a.post) e = awp_launch_post(pa, 0, s->stream);
     if (e == cudaSuccess && s->npts > 0 && ((steps + 1) % s->p.ntiskp_sgt == 0))
         e = awp_launch_sgt(sa, s->stream);
     return e;
@@ -1466,7 +1470,8 @@ static double part_bytes(const awp_solver *s, int part)
     switch (part) {
     case AWP_PART_VEL: return cells * (nc * 12 * 4.0 + mb);                          /* R 9 W 3 + d1 */
     case AWP_PART_FSVEL: return (double)p->nx * p->ny * (nc * (8 * 4.0) + 2 * mb);
-    case AWP_PART_STR: return cells * (nc * (15 * 4.0 + rcell) + (nmed - 1) * mb);
+    case AWP_PART_STR:
+        return cells * (nc * (15 * 4.0 + rcell) + (nmed - 1) * mb) + (s->staged_on ? part_bytes(s, AWP_PART_FSVEL) : 0.0);
     case AWP_PART_FUSED: return cells * (nc * (18 * 4.0 + rcell) + nmed * mb);
     case AWP_PART_PML_VEL:
     case AWP_PART_PML_STR: {
@@ -1497,7 +1502,7 @@ extern "C" awp_status awp_profile_steps(awp_solver *s, int nsteps, awp_kernel_ti
     else {
         parts[np++] = AWP_PART_VEL;
         if (p->npc == 1) parts[np++] = AWP_PART_PML_VEL;
-        parts[np++] = AWP_PART_FSVEL;
+        if (!s->staged_on) parts[np++] = AWP_PART_FSVEL;    /* part of the staged stress sweep */
         parts[np++] = AWP_PART_STR;
         if (p->npc == 1) parts[np++] = AWP_PART_PML_STR;
     }
@@ -2067,7 +2072,7 @@ extern "C" awp_status awp_reset(awp_solver *s)
     for (int q = 0; q < p->ncomp; q++)
         if (s->pml_split[q]) CU(cudaMemsetAsync(s->pml_split[q], 0, sizeof(float) * (size_t)s->pml_floats, s->stream));
     CU(cudaMemsetAsync(s->step, 0, sizeof(int), s->stream));
-    CU(cudaMemsetAsync(s->flag, 0, 2 * sizeof(int), s->stream));
+    CU(cudaMemsetAsync(s->flag, 0, 3 * sizeof(int), s->stream));
     CU(cudaStreamSynchronize(s->stream));
     s->steps_done = 0;
     s->started = 0;

@@ -36,6 +36,7 @@
 #include "awp_internal.h"
 #include "awp_kernels.h"
 #include "awp_stencil.cuh"
+#include "awp_post.cuh"
 
 #define ST_X 32                      /* tile width: one warp along x            */
 #define ST_Y 8                       /* tile rows                               */
@@ -373,6 +374,53 @@ __device__ __forceinline__ void str_issue(const AwpStagedStrMaps &maps, int q, i
     if (nve == 1) r_issue<TR>(maps, q, (unsigned char *)(sl + STR_ST + 6 * ST_PT), b, xp, j0 + 1, k + 1);
 }
 
+/* ---- the ends of a stress sweep ------------------------------------------ */
+
+/* Free-surface velocities of one column (fvelxy and fvelz, operator.f:246-306;
+ * k_fsvel's expressions).  Only the column's own stress update reads them (the
+ * z differences at k = nz-2 .. nz), so the thread that owns the column in the
+ * top chunk writes them before its levels and reads them back itself; a launch
+ * of their own cost about 3 us a step. */
+template <class TM>
+__device__ __forceinline__ void fs_velocity(const AwpGeom &g, float *u1, float *v1, float *w1, const TM *lam, const TM *mu,
+                                            const AwpMediaScale &sc, int i, int j)
+{
+    const int c = g.idx(i, j, g.nz), sy = g.px, sz = g.plane;
+    const float xl = 1.0f / Store<TM>::ld(lam, c, sc.inv[AM_LAM]);
+    const float xl2m = 2.0f / Store<TM>::ld(mu, c, sc.inv[AM_MU]) + xl;
+    const float u_fs = u1[c] - (w1[c] - w1[c - 1]);
+    const float v_fs = v1[c] - (w1[c + sy] - w1[c]);
+    const float u_fs_e = (i + 1 <= g.nx) ? (u1[c + 1] - (w1[c + 1] - w1[c])) : 0.0f;
+    const float v_fs_s = (j - 1 >= 1) ? (v1[c - sy] - (w1[c] - w1[c - sy])) : 0.0f;
+    const float w_fs = w1[c - sz] - __fmul_rn(xl / xl2m, (u_fs_e - u_fs) + (u1[c + 1] - u1[c]) + (v_fs - v_fs_s) + (v1[c] - v1[c - sy]));
+    u1[c + sz] = u_fs;
+    v1[c + sz] = v_fs;
+    w1[c + sz] = w_fs;
+}
+
+/* What a stress sweep does besides: the media arrays of fs_velocity, and the
+ * step's serial work once all its warps are done (done: their count, back at
+ * zero for the next launch; NULL: left to k_post). */
+struct StrEnds {
+    const void *lam, *mu;
+    int *done;
+    AwpPostArgs post;
+};
+
+/* the last of the grid's `warps` consumer warps runs step_post */
+__device__ __forceinline__ void str_finish(const StrEnds &e, int warps)
+{
+    if (!e.done) return;
+    __threadfence();                  /* this lane's stores before the count */
+    __syncwarp();
+    int n = 0;
+    if ((threadIdx.x & 31) == 0) n = atomicAdd(e.done, 1);
+    if (__shfl_sync(0xffffffffu, n, 0) != warps - 1) return;
+    __threadfence();
+    step_post(e.post, 0);
+    if ((threadIdx.x & 31) == 0) *e.done = 0;
+}
+
 /* work items: (x tile, y tile, z chunk, component); see split_item for the order.
  * RPT rows of the tile per consumer thread (ST_Y / RPT consumer warps): with
  * RPT = 2 a thread carries two independent cells per level. */
@@ -380,7 +428,8 @@ template <class TM, class TR, int UNR, int RPT>
 __global__ void __launch_bounds__(32 * (ST_Y / RPT + 1), 3)
 k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<AWP_MAX_COMP> cs, int ncomp, int qslow,
           const float *__restrict__ cx, const float *__restrict__ cy, const float *__restrict__ cz,
-          const float *__restrict__ tau, float dth, float dt, float dh1, AwpWork w, int nve, AwpMediaScale sc, int *err, AwpWait wt)
+          const float *__restrict__ tau, float dth, float dt, float dh1, AwpWork w, int nve, const __grid_constant__ AwpMediaScale sc, int *err, AwpWait wt,
+          const __grid_constant__ StrEnds ends)
 {
     constexpr int S = 2 + STR_D;      /* levels k-1 and k in use, STR_D in flight */
     constexpr int CW = ST_Y / RPT;    /* consumer warps */
@@ -429,7 +478,7 @@ k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<A
         staged_item(g, w, t, bx, by, k0, k1);
         const int i = bx * ST_X + 1 + tx;
         const int np = k1 - k0 + 2;   /* levels k0-1 .. k1 */
-        const float *U = tab[q].f[AF_U], *V = tab[q].f[AF_V], *W = tab[q].f[AF_W];
+        float *U = tab[q].f[AF_U], *V = tab[q].f[AF_V], *W = tab[q].f[AF_W];
         /* per row: column queues u, v at k+1, k+2 (k+3 loaded one level ahead), w at k-2, k+1 (k+2 ahead) */
         float up1[RPT], up2[RPT], vp1[RPT], vp2[RPT], wm2[RPT], wp1[RPT], cxy[RPT];
         bool live[RPT];
@@ -442,6 +491,8 @@ k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<A
             itxy[r] = ((j & 1) << 1) | (i & 1);
             up1[r] = up2[r] = vp1[r] = vp2[r] = wm2[r] = wp1[r] = cxy[r] = 0.f;
             if (live[r]) {
+                if (k1 == g.nz)
+                    fs_velocity(g, U, V, W, (const TM *)ends.lam, (const TM *)ends.mu, sc, i, j);
                 up1[r] = __ldg(&U[c + sz]); up2[r] = __ldg(&U[c + 2 * sz]);
                 vp1[r] = __ldg(&V[c + sz]); vp2[r] = __ldg(&V[c + 2 * sz]);
                 wm2[r] = __ldg(&W[c - 2 * sz]); wp1[r] = __ldg(&W[c + sz]);
@@ -458,7 +509,7 @@ k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<A
             for (int r = 0; r < RPT; ++r) {
                 const int c = cc + r * CW * sy;
                 up3[r] = vp3[r] = wp2[r] = 0.f;
-                if (live[r] && k < k1) { up3[r] = __ldg(&U[c + 3 * sz]); vp3[r] = __ldg(&V[c + 3 * sz]); wp2[r] = __ldg(&W[c + 2 * sz]); }
+                if (live[r] && k < k1) { up3[r] = __ldcg(&U[c + 3 * sz]); vp3[r] = __ldcg(&V[c + 3 * sz]); wp2[r] = __ldcg(&W[c + 2 * sz]); }
             }
             bool ok = true;
             if (k == k0) ok = mb_wait_or_abort(&full[usem % S], (usem / S) & 1, &abort_s, wt.ns);
@@ -524,6 +575,7 @@ k_str_tma(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<A
             }
         }
     }
+    str_finish(ends, gridDim.x * CW);
 }
 
 /* ---- components side by side in one work item -------------------------- */
@@ -550,7 +602,8 @@ template <class TM, class TR, int NCB, int STB_CS, int RPT>
 __global__ void __launch_bounds__(32 * (ST_Y / RPT + 1), 2)
 k_str_tmab(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<AWP_MAX_COMP> cs,
            const float *__restrict__ cx, const float *__restrict__ cy, const float *__restrict__ cz,
-           const float *__restrict__ tau, float dth, float dt, float dh1, AwpWork w, int nve, AwpMediaScale sc, int *err, AwpWait wt)
+           const float *__restrict__ tau, float dth, float dt, float dh1, AwpWork w, int nve, const __grid_constant__ AwpMediaScale sc, int *err, AwpWait wt,
+          const __grid_constant__ StrEnds ends)
 {
     constexpr int CW = ST_Y / RPT;    /* consumer warps */
     extern __shared__ unsigned char st_smem[];
@@ -643,7 +696,9 @@ k_str_tmab(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<
                 up1[r][q] = up2[r][q] = pu[r][q] = vp1[r][q] = vp2[r][q] = pv[r][q] = wp1[r][q] = pw[r][q] = 0.f;
                 wm2[r][q] = wm1[r][q] = um1[r][q] = vm1[r][q] = 0.f;
                 if (live[r]) {
-                    const float *U = tab[q].f[AF_U], *V = tab[q].f[AF_V], *W = tab[q].f[AF_W];
+                    float *U = tab[q].f[AF_U], *V = tab[q].f[AF_V], *W = tab[q].f[AF_W];
+                    if (k1 == g.nz)
+                        fs_velocity(g, U, V, W, (const TM *)ends.lam, (const TM *)ends.mu, sc, i, j);
                     up2[r][q] = __ldg(&U[c + sz]); pu[r][q] = __ldg(&U[c + 2 * sz]);
                     vp2[r][q] = __ldg(&V[c + sz]); pv[r][q] = __ldg(&V[c + 2 * sz]);
                     pw[r][q] = __ldg(&W[c + sz]);
@@ -688,9 +743,9 @@ k_str_tmab(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<
                     wp1[r][q] = pw[r][q];
                     pu[r][q] = pv[r][q] = pw[r][q] = 0.f;
                     if (live[r] && k < k1) {
-                        pu[r][q] = __ldg(&tab[q].f[AF_U][c + 3 * sz]);
-                        pv[r][q] = __ldg(&tab[q].f[AF_V][c + 3 * sz]);
-                        pw[r][q] = __ldg(&tab[q].f[AF_W][c + 2 * sz]);
+                        pu[r][q] = __ldcg(&tab[q].f[AF_U][c + 3 * sz]);
+                        pv[r][q] = __ldcg(&tab[q].f[AF_V][c + 3 * sz]);
+                        pw[r][q] = __ldcg(&tab[q].f[AF_W][c + 2 * sz]);
                     }
                 }
                 ok = mb_wait_or_abort(&cfull[uc % STB_CS], (uc / STB_CS) & 1, &abort_s, wt.ns);
@@ -754,6 +809,7 @@ k_str_tmab(const __grid_constant__ AwpStagedStrMaps maps, AwpGeom g, AwpCompSet<
             }
         }
     }
+    str_finish(ends, gridDim.x * CW);
 }
 
 #include "awp_pair.cuh"
@@ -923,6 +979,19 @@ static int staged_grid(const StagedSlots &sl, const AwpWork &w)
     return n < w.nitems ? n : w.nitems;
 }
 
+static StrEnds str_ends(const AwpStepArgs &s)
+{
+    StrEnds e;
+    memset(&e, 0, sizeof e);
+    e.lam = s.md.m[AM_LAM];
+    e.mu = s.md.m[AM_MU];
+    if (s.post) {
+        e.post = *s.post;
+        e.done = s.post_done;
+    }
+    return e;
+}
+
 static AwpCompSet<AWP_MAX_COMP> comp_set3(const AwpStepArgs &s)
 {
     AwpCompSet<AWP_MAX_COMP> cs;
@@ -960,7 +1029,7 @@ static cudaError_t launch_str_rpt(const AwpStaged *st, const AwpStepArgs &s, cud
     const AwpWork w = staged_work(s.g, ST_Y, s.kchunk_staged, s.ncomp, sl, 1.5);
     k_str_tma<TM, TR, UNR, RPT><<<staged_grid(sl, w), dim3(32, CW + 1), smem, stream>>>(st->sm, s.g, comp_set3(s), s.ncomp,
                                                                        s.staged_qslow, s.cx, s.cy, s.cz, s.tau,
-                                                                       s.dth, s.dt, s.dh1, w, s.nve, s.md.sc, s.kerr, awp_wait_of(s));
+                                                                       s.dth, s.dt, s.dh1, w, s.nve, s.md.sc, s.kerr, awp_wait_of(s), str_ends(s));
     return cudaGetLastError();
 }
 
@@ -975,7 +1044,7 @@ static cudaError_t launch_str_bc(const AwpStaged *st, const AwpStepArgs &s, cuda
     if (e != cudaSuccess) return e;
     const AwpWork w = staged_work(s.g, ST_Y, s.kchunk_staged, 1, sl, 1.0);
     k_str_tmab<TM, TR, NCB, CS, RPT><<<staged_grid(sl, w), dim3(32, CW + 1), smem, stream>>>(
-        st->sm, s.g, comp_set3(s), s.cx, s.cy, s.cz, s.tau, s.dth, s.dt, s.dh1, w, s.nve, s.md.sc, s.kerr, awp_wait_of(s));
+        st->sm, s.g, comp_set3(s), s.cx, s.cy, s.cz, s.tau, s.dth, s.dt, s.dh1, w, s.nve, s.md.sc, s.kerr, awp_wait_of(s), str_ends(s));
     return cudaGetLastError();
 }
 
