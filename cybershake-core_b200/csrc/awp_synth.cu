@@ -884,7 +884,8 @@ extern "C" awp_status awp_synth_run(awp_synth *s)
     cudaError_t e = cudaSuccess;
     e = e ? e : s->d_seis.reserve((size_t)nv * 3 * ntout);
     e = e ? e : s->h_seis.reserve((size_t)nv * 3 * ntout);
-    for (auto &sg : s->stage) {
+    for (size_t k = 0; k < 2 && k < chunks.size(); k++) {      /* a single chunk needs one stage */
+        Stage &sg = s->stage[k];
         e = e ? e : sg.gt.reserve((size_t)max_terms);
         e = e ? e : sg.ct.reserve((size_t)max_terms);
         e = e ? e : sg.stf.reserve((size_t)max_stf + 8);
