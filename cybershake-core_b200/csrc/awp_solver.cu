@@ -98,8 +98,7 @@ struct awp_solver {
     size_t stagger;                  /* base-address offset step of the field arrays */
     int nstag;
     struct { void *user, *raw; } stag[AWP_MAX_FIELDS];   /* field arrays: pointer in use, block */
-    int kchunk_staged;               /* z levels per staged work item       */
-    int kchunk_auto;                 /* not set by anyone: each sweep picks its own (awp_staged.cu) */
+    int kchunk_staged;               /* z levels per staged work item; 0: each sweep picks its own (awp_staged.cu) */
     int staged_qslow;                /* staged items: component slowest     */
     int staged_rpt;                  /* staged stress sweep rows per thread */
     int staged_rpt_vel;              /* staged velocity sweep rows per thread */
@@ -704,16 +703,8 @@ extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
     s->kchunk = choose_kchunk(s->g, 1, s->ty);
     s->kchunk_sweep = choose_kchunk(s->g, 0, s->ty == 4 ? 4 : 8);
     {
-        /* z chunks: each sweep picks its own from the grid and its resident
-         * blocks unless told otherwise; what awp_get_tuning reports then is
-         * about 40 levels, split evenly */
-        int kc = env_int("AWP_TUNE_KSTAGE", 0);
-        s->kchunk_auto = kc <= 0;
-        if (kc <= 0) {
-            const int nch = (s->g.nz + 39) / 40;
-            kc = (s->g.nz + nch - 1) / nch;
-        }
-        s->kchunk_staged = kc < 8 ? 8 : (kc > s->g.nz ? s->g.nz : kc);
+        const int kc = env_int("AWP_TUNE_KSTAGE", 0);
+        s->kchunk_staged = kc <= 0 ? 0 : (kc < 8 ? 8 : (kc > s->g.nz ? s->g.nz : kc));
         s->staged_qslow = env_int("AWP_TUNE_QSLOW", 1) != 0;
         /* stress sweep rows per consumer thread: two pay off once three
          * components share the sweep with FP32 memory variables */
@@ -1237,7 +1228,7 @@ static void fill_args(awp_solver *s, int steps, AwpStepArgs &a, AwpPostArgs &pa,
     a.ty = s->ty;
     a.unroll = s->unroll;
     a.staged = s->staged_on ? s->staged : NULL;
-    a.kchunk_staged = s->kchunk_auto ? 0 : s->kchunk_staged;
+    a.kchunk_staged = s->kchunk_staged;
     a.staged_qslow = s->staged_qslow;
     a.staged_rpt = s->staged_rpt;
     a.staged_batch = s->staged_batch;
@@ -2255,9 +2246,9 @@ extern "C" awp_status awp_set_tuning(awp_solver *s, const awp_tuning *t)
 {
     if (!s || !t) return set_err(AWP_ERR_PARAM, "awp_set_tuning: null argument");
     const int nz = s->g.nz, kmax = nz > 8 ? nz : 8;
-    if (t->kchunk_staged < 8 || t->kchunk_staged > kmax || t->kchunk < 8 || t->kchunk > kmax ||
-        t->kchunk_sweep < 8 || t->kchunk_sweep > kmax)
-        return set_err(AWP_ERR_PARAM, "awp_set_tuning: z levels per work item must be 8..%d", kmax);
+    if ((t->kchunk_staged != 0 && (t->kchunk_staged < 8 || t->kchunk_staged > kmax)) || t->kchunk < 8 ||
+        t->kchunk > kmax || t->kchunk_sweep < 8 || t->kchunk_sweep > kmax)
+        return set_err(AWP_ERR_PARAM, "awp_set_tuning: z levels per work item must be 8..%d (staged sweeps: or 0)", kmax);
     if ((t->staged_qslow != 0 && t->staged_qslow != 1) || (t->staged_rpt != 1 && t->staged_rpt != 2) ||
         (t->staged_rpt_vel != 1 && t->staged_rpt_vel != 2) || (t->unroll != 1 && t->unroll != 2) ||
         (t->ty != 4 && t->ty != 8 && t->ty != 16) || t->staged_batch < 0 || t->staged_batch > 3 || t->sm_limit < 0)
@@ -2265,7 +2256,6 @@ extern "C" awp_status awp_set_tuning(awp_solver *s, const awp_tuning *t)
                        "0-3, sm_limit >= 0");
     CU(cudaSetDevice(s->p.device));
     CU(cudaStreamSynchronize(s->stream));   /* no captured step in flight when its graph goes */
-    if (s->kchunk_staged != t->kchunk_staged) s->kchunk_auto = 0;
     s->kchunk_staged = t->kchunk_staged;
     s->staged_qslow = t->staged_qslow;
     s->staged_rpt = t->staged_rpt;
@@ -2280,7 +2270,8 @@ extern "C" awp_status awp_set_tuning(awp_solver *s, const awp_tuning *t)
     return AWP_OK;
 }
 
-/* "nx ny nz ncomp precision nve stepper gpu-model" */
+/* "shapes2 nx ny nz ncomp precision nve stepper gpu-model"; the first word names the meaning of the record,
+ * so that lines written when it was another (no automatic z split) are not matched */
 static void tune_key(const awp_params *p, int stepper, char *key, size_t n)
 {
     cudaDeviceProp prop;
@@ -2290,7 +2281,7 @@ static void tune_key(const awp_params *p, int stepper, char *key, size_t n)
         for (char *c = model; *c; ++c)
             if (*c == ' ') *c = '_';
     }
-    snprintf(key, n, "%d %d %d %d %d %d %d %s", p->nx, p->ny, p->nz, p->ncomp, (int)p->precision, p->nve, stepper,
+    snprintf(key, n, "shapes2 %d %d %d %d %d %d %d %s", p->nx, p->ny, p->nz, p->ncomp, (int)p->precision, p->nve, stepper,
              model);
 }
 
@@ -2403,7 +2394,8 @@ extern "C" awp_status awp_autotune(const awp_params *pin, const float *media, in
         int vals[6], nv = 0;
         switch (fields[fi]) {
         case F_KSTAGE:
-            for (int target : {24, 32, 40, 48, 64}) {
+            /* against the automatic split (0), whose chunks are 5 to 30 levels on grids up to 400^2 x 200 */
+            for (int target : {8, 12, 16, 24, 40, 64}) {
                 const int nch = (p.nz + target - 1) / target;
                 int kc = (p.nz + nch - 1) / nch;
                 kc = kc < 8 ? 8 : kc;
@@ -2412,12 +2404,19 @@ extern "C" awp_status awp_autotune(const awp_params *pin, const float *media, in
                 if (!dup) vals[nv++] = kc;
             }
             break;
-        /* the side-by-side sweeps ignore rows per thread and component order */
+        /* only what selects another kernel or order (launch_str_tr): the staged stress sweep has rows per
+         * thread and an unroll for FP32 media, one component per item, and the unroll with one row only */
         case F_RPT:
-            if (!((cur.staged_batch & 1) && p.ncomp >= 2)) vals[nv++] = 3 - cur.staged_rpt;
+            if (s->store == AWP_STORE_F32 && !((cur.staged_batch & 1) && p.ncomp >= 2)) vals[nv++] = 3 - cur.staged_rpt;
             break;
-        case F_UNROLL: vals[nv++] = 3 - cur.unroll; break;
-        case F_QSLOW: vals[nv++] = 1 - cur.staged_qslow; break;
+        case F_UNROLL:
+            if (stepper == AWP_KERNEL_TWO_SWEEP || (s->store == AWP_STORE_F32 && cur.staged_rpt == 1 &&
+                                                    !((cur.staged_batch & 1) && p.ncomp >= 2)))
+                vals[nv++] = 3 - cur.unroll;
+            break;
+        case F_QSLOW:
+            if (p.ncomp >= 2) vals[nv++] = 1 - cur.staged_qslow;
+            break;
         case F_BATCH: vals[nv++] = cur.staged_batch ^ 1; break;
         case F_TY:
             for (int ty : {4, 8, 16})

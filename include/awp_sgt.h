@@ -322,7 +322,9 @@ awp_status awp_profile_steps(awp_solver *s, int nsteps, awp_kernel_times *out);
  * awp_set_tuning replaces them at any point of a solve (a captured time-loop
  * graph is rebuilt on the next step). */
 typedef struct {
-    int kchunk_staged;       /* staged sweeps: z levels per work item (8..nz)          */
+    int kchunk_staged;       /* staged sweeps: z levels per work item (8..nz); 0, the
+                                default: each sweep splits nz by its tiles and its
+                                resident blocks                                        */
     int staged_qslow;        /* staged sweeps: 1 = one component over all tiles first  */
     int staged_rpt;          /* staged stress sweep, one component per item: tile rows
                                 per thread (1, 2)                                      */

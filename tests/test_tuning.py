@@ -89,6 +89,35 @@ def test_set_tuning_rejects_bad_shapes():
     assert s.tuning().as_dict() == t.as_dict()      # a rejected tuning changes nothing
 
 
+def test_automatic_z_split_is_a_value_of_its_own(tmp_path):
+    """kchunk_staged = 0 (the default) is the automatic split: a record read,
+    replaced and written back is the same record again, any explicit chunk is
+    kept as asked for, and a record from a cache of another meaning is not
+    used."""
+    c = Case(nx=40, ny=32, nz=30, nt=30, igreen=(1, 2), srcs=[[(20, 16, 6)], [(18, 15, 9)]])
+    s = solver_for(c, "staged")
+    t0 = s.tuning()
+    assert t0.kchunk_staged == 0
+    for kc in (8, 30, 0, 17):
+        s.set_tuning(variant(t0, kchunk_staged=kc))
+        assert s.tuning().kchunk_staged == kc
+        s.run(6)
+    s.set_tuning(t0)
+    assert s.tuning().as_dict() == t0.as_dict()
+    s.run(c.nt)
+    for q in range(2):
+        assert_same_state(s, c.oracle(q), q)
+    # an entry written before the automatic split had a value: not matched
+    p = awpsgt.make_params(c.nx, c.ny, c.nz, c.dh, c.dt, c.nt, igreen=c.igreen, kernel="staged", **c.kw())
+    cache = tmp_path / "tune.txt"
+    awpsgt.autotune(p, c.media, trial_steps=4, cache=str(cache))
+    new = cache.read_text().split()
+    old = new[1:9] + ["29", "1", "1", "1", "2", "8", "16", "8", "1", "0.001"]
+    cache.write_text(" ".join(old) + "\n")
+    t, rate = awpsgt.autotune(p, c.media, trial_steps=4, cache=str(cache))
+    assert rate > 0.001 and t.sm_limit == 0
+
+
 @pytest.mark.parametrize("kernel", ["staged", "fused"])
 def test_autotune_and_cache(kernel, tmp_path):
     c = Case(nx=96, ny=80, nz=72, nt=10, igreen=(1, 2))
