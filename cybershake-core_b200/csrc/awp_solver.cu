@@ -1561,9 +1561,11 @@ extern "C" awp_status awp_get_sgt_rwg(awp_solver *s, int comp, int z_source, flo
     /* from the block cache: allocating and freeing device memory here cost up
      * to 7 ms a call in a process with other solvers */
     float *tmp = NULL;
-    cudaError_t e = blk_alloc(s->p.device, (void **)&tmp, sizeof(float) * (size_t)s->sgt_file_floats);
-    if (e != cudaSuccess) return set_err(AWP_ERR_CUDA, "awp_get_sgt_rwg: %s", cudaGetErrorString(e));
-    e = awp_launch_sgt_rwg(s->sgt_file[comp], tmp, s->npts, s->nt_file, z_source != 0, s->stream);
+    const size_t bytes = sizeof(float) * (size_t)s->sgt_file_floats;
+    const awp_status st = dalloc(s, (void **)&tmp, bytes);
+    if (st != AWP_OK) return st;
+    s->device_bytes -= (double)bytes;                 /* not part of the solver's state */
+    cudaError_t e = awp_launch_sgt_rwg(s->sgt_file[comp], tmp, s->npts, s->nt_file, z_source != 0, s->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(out, tmp, sizeof(float) * (size_t)s->sgt_file_floats, cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);

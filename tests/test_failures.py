@@ -61,3 +61,24 @@ def test_failed_allocation_is_oom_and_releases_everything(monkeypatch, nth):
     assert np.abs(s.sgt()).max() > 0
     s.close()
     assert awpsgt.device_memory(0)[0] == live0
+
+
+def test_failed_sgt_staging_is_oom(monkeypatch):
+    """The staging block of awp_get_sgt_rwg is the first allocation after a
+    solve is set up: made to fail there, the call reports AWP_ERR_OOM and the
+    next one works."""
+    c = Case(nt=20)
+    want = c.gpu().sgt_rwg(0, z_source=False)
+    for nth in range(10, 200):
+        monkeypatch.setenv("AWP_TEST_FAIL_ALLOC", str(nth))
+        try:
+            s = c.gpu()
+        except awpsgt.AwpError as e:
+            assert awpsgt.STATUS[e.status] == "AWP_ERR_OOM"
+            continue
+        with pytest.raises(awpsgt.AwpError) as e:
+            s.sgt_rwg(0, z_source=False)
+        assert awpsgt.STATUS[e.value.status] == "AWP_ERR_OOM"
+        assert np.array_equal(s.sgt_rwg(0, z_source=False), want)
+        return
+    raise AssertionError("no allocation of a solve was made to fail")
