@@ -2297,6 +2297,7 @@ static int tune_cache_get(const char *path, const char *key, awp_tuning *t, doub
     while (fgets(line, sizeof line, f)) {
         if (strncmp(line, key, kl) != 0 || line[kl] != ' ') continue;
         awp_tuning u;
+        memset(&u, 0, sizeof u);              /* sm_limit is not kept in the file */
         double r = 0.0;
         if (sscanf(line + kl, "%d %d %d %d %d %d %d %d %d %lf", &u.kchunk_staged, &u.staged_qslow, &u.staged_rpt,
                    &u.staged_rpt_vel, &u.unroll, &u.ty, &u.kchunk, &u.kchunk_sweep, &u.staged_batch, &r) == 10) {

@@ -130,6 +130,7 @@ def test_autotune_and_cache(kernel, tmp_path):
     # the second call reads the cache (same result, no new line)
     t2, rate2 = awpsgt.autotune(p, c.media, trial_steps=4, cache=cache)
     assert t2.as_dict() == t.as_dict() and rate2 == pytest.approx(rate, rel=1e-5)
+    assert t2.sm_limit == 0            # not in the file: every SM
     assert len(open(cache).read().splitlines()) == 1
     # a homogeneous trial of another grid is a new key
     p2 = awpsgt.make_params(c.nx, c.ny, 64, c.dh, c.dt, c.nt, igreen=c.igreen, kernel=kernel, **c.kw())
