@@ -416,6 +416,7 @@ __device__ __forceinline__ void str_finish(const StrEnds &e, int warps)
     int n = 0;
     if ((threadIdx.x & 31) == 0) n = atomicAdd(e.done, 1);
     if (__shfl_sync(0xffffffffu, n, 0) != warps - 1) return;
+    __syncwarp();                     /* lane 0's count before every lane's loads (a shuffle orders no memory) */
     __threadfence();
     step_post(e.post, 0);
     if ((threadIdx.x & 31) == 0) *e.done = 0;
