@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -30,6 +31,9 @@
 #include "../../include/awp_sgt.h"
 
 extern "C" void awp_set_error_text(const char *msg);
+/* awp_solver.cu: rows padded to whole 128-byte lines (pad = 1) or not */
+int64_t awp_footprint_rows(const awp_params *p, int npts, int pad);
+awp_status awp_create_rows(const awp_params *p, int pad, awp_solver **out);
 
 namespace {
 
@@ -43,6 +47,7 @@ struct Req {
     double cells = 0;      /* cells x components: work of one step */
     double work = 0;       /* cells x components x steps           */
     int sm_share = 0;      /* SMs its grids are sized for (0 = all)  */
+    int pad = 0;           /* padded rows (info.footprint counts them) */
 };
 
 awp_status fail(awp_status st, const char *msg)
@@ -119,7 +124,8 @@ void awp_server::end(Req *r, int state, awp_status st)
 awp_status awp_server::build(Req *r)
 {
     awp_solver *s = nullptr;
-    awp_status st = awp_create(&r->rq.params, &s);
+    awp_status st = awp_create_rows(&r->rq.params, r->pad, &s);
+    if (st == AWP_ERR_OOM && r->pad) st = awp_create_rows(&r->rq.params, 0, &s);
     if (st == AWP_OK) st = awp_load_media(s, r->rq.media);
     for (int q = 0; q < r->rq.params.ncomp && st == AWP_OK; q++)
         st = awp_set_source(s, q, r->rq.nsrc[q], r->rq.src_xyz[q], r->rq.stf[q]);
@@ -333,7 +339,11 @@ extern "C" awp_status awp_submit(awp_server *sv, const awp_request *rq, int64_t 
     r->rq = *rq;
     memset(&r->info, 0, sizeof r->info);
     r->info.state = AWP_REQ_QUEUED;
-    r->info.footprint = fp;
+    /* padded rows, unless fewer solves of this size could be resident with them */
+    const int64_t fpad = awp_footprint_rows(&rq->params, rq->npts, 1);
+    auto resident = [&](int64_t f) { return std::min<int64_t>(sv->max_active, sv->budget / std::max<int64_t>(f, 1)); };
+    r->pad = resident(fpad) == resident(fp);
+    r->info.footprint = r->pad ? fpad : fp;
     const awp_params &p = rq->params;
     r->cells = (double)p.nx * p.ny * p.nz * (p.ncomp > 0 ? p.ncomp : 1);
     r->work = r->cells * p.nt;

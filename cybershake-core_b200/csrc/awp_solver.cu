@@ -97,7 +97,10 @@ struct awp_solver {
     int nkin[AWP_MAX_COMP];
     size_t stagger;                  /* base-address offset step of the field arrays */
     int nstag;
-    struct { void *user, *raw; } stag[AWP_MAX_FIELDS];   /* field arrays: pointer in use, block */
+    struct { void *user, *raw; int esize; } stag[AWP_MAX_FIELDS];   /* field arrays: pointer in use, block */
+    int lent;                        /* a field pointer was handed out: the arrays stay where they are */
+    int wrote;                       /* a wavefield was set from outside since the arrays were zeroed */
+    int lost;                        /* narrow_rows failed halfway: no arrays */
     int kchunk_staged;               /* z levels per staged work item; 0: each sweep picks its own (awp_staged.cu) */
     int staged_qslow;                /* staged items: component slowest     */
     int staged_rpt;                  /* staged stress sweep rows per thread */
@@ -178,12 +181,14 @@ extern "C" void awp_params_default(awp_params *p)
     p->npc = 0; p->pht = 0.1f;
 }
 
-static AwpGeom make_geom(const awp_params *p)
+/* pad: rows of a multiple of 32 cells (awp_internal.h), unless they pass the
+ * 32-bit index range; else of 8 */
+static AwpGeom make_geom(const awp_params *p, int pad)
 {
     AwpGeom g;
     g.nx = p->nx; g.ny = p->ny; g.nz = p->nz;
     g.px = ((p->nx + AWP_XO + 2) + 31) / 32 * 32;
-    if ((int64_t)g.px * (p->ny + 4) * (p->nz + 4) >= (int64_t)1 << 31) g.px = ((p->nx + AWP_XO + 2) + 7) / 8 * 8;
+    if (!pad || (int64_t)g.px * (p->ny + 4) * (p->nz + 4) >= (int64_t)1 << 31) g.px = ((p->nx + AWP_XO + 2) + 7) / 8 * 8;
     g.py = p->ny + 4;
     g.plane = g.px * g.py;
     g.vol = (int64_t)g.plane * (p->nz + 4);
@@ -263,9 +268,9 @@ static int choose_kchunk(const AwpGeom &g, int fused, int ty)
     return kc;
 }
 
-extern "C" int64_t awp_footprint_bytes(const awp_params *p, int npts)
+int64_t awp_footprint_rows(const awp_params *p, int npts, int pad)
 {
-    AwpGeom g = make_geom(p);
+    AwpGeom g = make_geom(p, pad);
     const int nc = p->ncomp < 1 ? 1 : p->ncomp;
     const int st = store_of(p);
     const double mb = media_word(st);
@@ -283,6 +288,8 @@ extern "C" int64_t awp_footprint_bytes(const awp_params *p, int npts)
     b += 64ll << 20;   /* media staging slab + small buffers */
     return b;
 }
+
+extern "C" int64_t awp_footprint_bytes(const awp_params *p, int npts) { return awp_footprint_rows(p, npts, 0); }
 
 /* sponge factor of a face, cerjan.f:52 and :76 (float arithmetic) */
 static float crj_low(float alpha, int nd, int g)
@@ -398,6 +405,20 @@ static void blk_trim(int dev)
     for (void *p : out) cudaFree(p);
 }
 
+/* cudaMalloc; AWP_TEST_DEVICE_BYTES (tests) makes it fail once live and idle
+ * blocks would pass that many bytes, as on a device of that size */
+static cudaError_t blk_malloc(int dev, void **ptr, size_t bytes)
+{
+    if (const char *cap = getenv("AWP_TEST_DEVICE_BYTES")) {
+        std::lock_guard<std::mutex> lk(g_blk_mu);
+        size_t held = g_blk_idle_bytes[dev];
+        for (const auto &kv : g_blk_live)
+            if (kv.second.dev == dev) held += kv.second.bytes;
+        if (held + bytes > (size_t)strtoull(cap, NULL, 10)) return cudaErrorMemoryAllocation;
+    }
+    return cudaMalloc(ptr, bytes);
+}
+
 static cudaError_t blk_alloc(int dev, void **ptr, size_t bytes)
 {
     {
@@ -412,11 +433,11 @@ static cudaError_t blk_alloc(int dev, void **ptr, size_t bytes)
             return cudaSuccess;
         }
     }
-    cudaError_t e = cudaMalloc(ptr, bytes);
+    cudaError_t e = blk_malloc(dev, ptr, bytes);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         blk_trim(dev);
-        e = cudaMalloc(ptr, bytes);
+        e = blk_malloc(dev, ptr, bytes);
     }
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> lk(g_blk_mu);
@@ -439,6 +460,16 @@ static void blk_free(void *p)
                 return;
             }
         }
+    }
+    cudaFree(p);
+}
+
+/* back to the driver instead of the cache */
+static void blk_drop(void *p)
+{
+    {
+        std::lock_guard<std::mutex> lk(g_blk_mu);
+        g_blk_live.erase(p);
     }
     cudaFree(p);
 }
@@ -498,6 +529,7 @@ static awp_status dalloc_field(awp_solver *s, void **ptr, size_t bytes, int esiz
         if (!s->stag[n].raw) {
             *ptr = s->stag[n].user = (char *)raw + off;
             s->stag[n].raw = raw;
+            s->stag[n].esize = esize;
             break;
         }
     s->nstag++;
@@ -548,7 +580,7 @@ static awp_status check_params(const awp_params *p)
         int ig = p->igreen[q];
         if (!(ig == -2 || ig == -1 || (ig >= 1 && ig <= 6))) return set_err(AWP_ERR_PARAM, "IGREEN %d not supported", ig);
     }
-    AwpGeom g = make_geom(p);
+    AwpGeom g = make_geom(p, 0);
     if (g.vol >= (int64_t)1 << 31) return set_err(AWP_ERR_PARAM, "grid too large for 32-bit field indexing");
     return AWP_OK;
 }
@@ -570,9 +602,121 @@ static awp_status alloc_media32(awp_solver *s)
     return AWP_OK;
 }
 
-extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
+static void drop_graphs(awp_solver *s)
 {
-    NvtxScope nvtx_("awp_create");
+    for (int b = 0; b < 2; b++)
+        if (s->graph[b]) {
+            cudaGraphExecDestroy(s->graph[b]);
+            s->graph[b] = NULL;
+        }
+}
+
+/* Memory has run out before the first step: the fields move to rows of a
+ * multiple of 8 cells and the padding goes back to the driver.  Wavefields
+ * that nobody has written are all zero: they are released first, so that the
+ * media have room for their copies, and allocated again at the end.  Otherwise
+ * array after array is copied, which needs room for one more; without that,
+ * or when the rows are not padded or a field pointer has been handed out,
+ * nothing changes.  (If another thread takes the room in between, the arrays
+ * are gone and the solver answers AWP_ERR_OOM from then on.) */
+static awp_status narrow_rows(awp_solver *s)
+{
+    const AwpGeom o = s->g, g = make_geom(&s->p, 0);
+    if (g.px == o.px || s->started || s->lent) return AWP_ERR_OOM;
+    CU(cudaStreamSynchronize(s->stream));
+    drop_graphs(s);
+    awp_staged_destroy(s->staged);
+    s->staged = NULL;
+    struct Array {
+        void *user, *raw;
+        int esize, wave;
+        std::vector<void **> refs;                /* where the solver keeps the pointer */
+    };
+    std::vector<Array> old;
+    for (int wave = 0; wave < 2; wave++)          /* media first */
+        for (int k = 0; k < AWP_MAX_FIELDS; k++) {
+            if (!s->stag[k].raw) continue;
+            Array a{s->stag[k].user, s->stag[k].raw, s->stag[k].esize, 1, {}};
+            for (int m = 0; m < AM_N; m++) {
+                if (s->md.m[m] == a.user) a.wave = 0, a.refs.push_back((void **)&s->md.m[m]);
+                if (s->mdt.m[m] == a.user) a.wave = 0, a.refs.push_back(&s->mdt.m[m]);
+            }
+            for (int b = 0; b < 2; b++)
+                for (int q = 0; q < AWP_MAX_COMP; q++)
+                    for (int f = 0; f < AWP_NF_ARRAYS; f++)
+                        if (s->comp[b][q].f[f] == a.user) a.refs.push_back((void **)&s->comp[b][q].f[f]);
+            if (a.wave == wave) old.push_back(a);
+        }
+    auto drop = [&](Array &a) {
+        for (int k = 0; k < AWP_MAX_FIELDS; k++)
+            if (s->stag[k].raw == a.raw) s->stag[k].raw = NULL;
+        s->device_bytes -= (double)((size_t)o.vol * a.esize + (size_t)((char *)a.user - (char *)a.raw));
+        blk_drop(a.raw);
+        a.raw = NULL;
+        s->lost = 1;                              /* until every array is back */
+    };
+    if (!s->wrote)
+        for (Array &a : old)
+            if (a.wave) drop(a);
+    awp_status st = AWP_OK;
+    cudaError_t e = cudaSuccess;
+    for (Array &a : old) {
+        const size_t es = (size_t)a.esize, bytes = (size_t)g.vol * es, rows = (size_t)o.py * (size_t)(o.nz + 4);
+        void *to = NULL;
+        if ((st = dalloc_field(s, &to, bytes, a.esize)) != AWP_OK) break;
+        if (a.raw) e = cudaMemcpy2DAsync(to, g.px * es, a.user, o.px * es, g.px * es, rows, cudaMemcpyDeviceToDevice, s->stream);
+        else e = cudaMemsetAsync(to, 0, bytes, s->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+        if (e != cudaSuccess) { dfree_field(s, to); break; }
+        if (a.raw) drop(a);
+        for (void **r : a.refs) *r = to;
+        a.refs.clear();
+    }
+    if (!s->lost) return st != AWP_OK ? st : e != cudaSuccess ? AWP_ERR_CUDA : AWP_OK;
+    s->g = g;
+    s->pml_args.g = g;
+    for (int q = 0; q < s->p.ncomp; q++) s->pml_args.comp[q] = s->comp[0][q];
+    if (s->p.npc == 1) awp_pml_boxes(s->pml_args);
+    if (s->npts > 0) {
+        std::vector<int> idx((size_t)s->npts);
+        if (e == cudaSuccess) e = cudaMemcpy(idx.data(), s->pt_idx, sizeof(int) * idx.size(), cudaMemcpyDeviceToHost);
+        for (int &c : idx) c = c / o.px * g.px + c % o.px;       /* planes have the same number of rows */
+        if (e == cudaSuccess) e = cudaMemcpy(s->pt_idx, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice);
+    }
+    if (st == AWP_OK && e == cudaSuccess) {
+        s->lost = 0;
+        return AWP_OK;
+    }
+    for (Array &a : old) {                        /* arrays that did not get through: forget them */
+        if (a.raw) drop(a);
+        for (void **r : a.refs) *r = NULL;
+    }
+    s->media_loaded = 0;
+    return AWP_ERR_OOM;
+}
+
+/* refuses work on a solver whose arrays were lost (narrow_rows) */
+static awp_status check_alive(const awp_solver *s)
+{
+    return s->lost ? set_err(AWP_ERR_OOM, "the solver's arrays were lost when device memory ran out") : AWP_OK;
+}
+
+/* a set-up call that runs out of device memory is tried again without padding */
+template <class Call>
+static awp_status with_room(awp_solver *s, Call call)
+{
+    awp_status st = call();
+    if (st != AWP_ERR_OOM) return st;
+    char text[sizeof g_err];
+    memcpy(text, g_err, sizeof text);
+    if (narrow_rows(s) == AWP_OK) return call();
+    memcpy(g_err, text, sizeof text);
+    return st;
+}
+
+/* a solver with padded rows or without (make_geom) */
+awp_status awp_create_rows(const awp_params *pin, int pad, awp_solver **out)
+{
     *out = NULL;
     awp_status st = check_params(pin);
     if (st != AWP_OK) return st;
@@ -581,7 +725,7 @@ extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
     if (!s) return set_err(AWP_ERR_OOM, "host allocation failed");
     memset(s, 0, sizeof *s);
     s->p = *pin;
-    s->g = make_geom(pin);
+    s->g = make_geom(pin, pad);
     s->withhold = env_int("AWP_TEST_TMA_WITHHOLD", -1);
     {
         const int us = env_int("AWP_TEST_WAIT_US", 0);
@@ -729,6 +873,17 @@ extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
     return AWP_OK;
 }
 
+extern "C" awp_status awp_create(const awp_params *pin, awp_solver **out)
+{
+    NvtxScope nvtx_("awp_create");
+    awp_status st = awp_create_rows(pin, 1, out);
+    if (st == AWP_ERR_OOM && make_geom(pin, 1).px != make_geom(pin, 0).px) {
+        blk_trim(pin->device);                        /* the first try's blocks: too large to be a help */
+        st = awp_create_rows(pin, 0, out);
+    }
+    return st;
+}
+
 extern "C" awp_status awp_destroy(awp_solver *s)
 {
     if (!s) return AWP_OK;
@@ -873,12 +1028,11 @@ struct StageLease {
 
 /* direct != NULL: the media are already in page-locked host memory and are
  * copied from there slab by slab, without staging */
-static awp_status load_media_common(awp_solver *s, slab_reader rd, void *ctx, int rwg_nx = 0, int rwg_ny = 0,
-                                    const float *direct = NULL)
+static awp_status load_media_once(awp_solver *s, slab_reader rd, void *ctx, int rwg_nx, int rwg_ny, const float *direct)
 {
-    NvtxScope nvtx_("awp_load_media");
     const awp_params *p = &s->p;
     CU(cudaSetDevice(p->device));
+    if (s->lost) return check_alive(s);
     if (s->started) return set_err(AWP_ERR_STATE, "media must be loaded before the first step (or after awp_reset)");
     awp_status ast = alloc_media32(s);
     if (ast != AWP_OK) return ast;
@@ -966,6 +1120,14 @@ static awp_status load_media_common(awp_solver *s, slab_reader rd, void *ctx, in
         if (st != AWP_OK) return st;
     }
     return finish_media(s);
+}
+
+/* all its device memory is had before the first read, so a second try reads from the start too */
+static awp_status load_media_common(awp_solver *s, slab_reader rd, void *ctx, int rwg_nx = 0, int rwg_ny = 0,
+                                    const float *direct = NULL)
+{
+    NvtxScope nvtx_("awp_load_media");
+    return with_room(s, [&] { return load_media_once(s, rd, ctx, rwg_nx, rwg_ny, direct); });
 }
 
 struct mem_ctx { const float *base; };
@@ -1101,9 +1263,8 @@ extern "C" awp_status awp_reformat_velocity(int nx, int ny, int nz, const char *
 /* sources and points                                                  */
 /* ------------------------------------------------------------------ */
 
-extern "C" awp_status awp_set_source(awp_solver *s, int comp, int nsrc, const int *xyz, const float *stf)
+static awp_status set_source_once(awp_solver *s, int comp, int nsrc, const int *xyz, const float *stf)
 {
-    if (!s) return set_err(AWP_ERR_PARAM, "null solver");
     const awp_params *p = &s->p;
     if (comp < 0 || comp >= p->ncomp) return set_err(AWP_ERR_PARAM, "component %d out of range", comp);
     if (nsrc < 0 || (nsrc > 0 && (!xyz || !stf))) return set_err(AWP_ERR_PARAM, "bad source arrays");
@@ -1115,8 +1276,7 @@ extern "C" awp_status awp_set_source(awp_solver *s, int comp, int nsrc, const in
         if (xyz[3 * m + 2] < 1 || xyz[3 * m + 2] > p->nz) return set_err(AWP_ERR_PARAM, "Z source coordinate %d is outside range 1-%d", xyz[3 * m + 2], p->nz);
     }
     CU(cudaSetDevice(p->device));
-    for (int b = 0; b < 2; b++)
-        if (s->graph[b]) { cudaGraphExecDestroy(s->graph[b]); s->graph[b] = NULL; }
+    drop_graphs(s);
     dfree(s, s->src_ijk[comp]); s->src_ijk[comp] = NULL;
     dfree(s, s->src_stf[comp]); s->src_stf[comp] = NULL;
     dfree(s, s->kin[comp]); s->kin[comp] = NULL;
@@ -1159,10 +1319,23 @@ extern "C" awp_status awp_set_source(awp_solver *s, int comp, int nsrc, const in
     return st;
 }
 
-extern "C" awp_status awp_set_points(awp_solver *s, int npts, const int *xyz)
+extern "C" awp_status awp_set_source(awp_solver *s, int comp, int nsrc, const int *xyz, const float *stf)
 {
-    NvtxScope nvtx_("awp_set_points");
     if (!s) return set_err(AWP_ERR_PARAM, "null solver");
+    return with_room(s, [&] { return set_source_once(s, comp, nsrc, xyz, stf); });
+}
+
+static void set_points_release(awp_solver *s)
+{
+    dfree(s, s->pt_idx); s->pt_idx = NULL;
+    dfree(s, s->sg); s->sg = NULL;
+    for (int q = 0; q < AWP_MAX_COMP; q++) { dfree(s, s->sgt_file[q]); s->sgt_file[q] = NULL; }
+    s->npts = 0;
+    s->sgt_file_floats = 0;
+}
+
+static awp_status set_points_once(awp_solver *s, int npts, const int *xyz)
+{
     const awp_params *p = &s->p;
     if (npts < 0 || (npts > 0 && !xyz)) return set_err(AWP_ERR_PARAM, "bad point arrays");
     if (s->started) return set_err(AWP_ERR_STATE, "points must be set before the first step");
@@ -1172,11 +1345,8 @@ extern "C" awp_status awp_set_points(awp_solver *s, int npts, const int *xyz)
             return set_err(AWP_ERR_PARAM, "SGT point %d (%d,%d,%d) outside the grid", n, xyz[3 * n], xyz[3 * n + 1], xyz[3 * n + 2]);
     }
     CU(cudaSetDevice(p->device));
-    for (int b = 0; b < 2; b++)
-        if (s->graph[b]) { cudaGraphExecDestroy(s->graph[b]); s->graph[b] = NULL; }
-    dfree(s, s->pt_idx); s->pt_idx = NULL;
-    dfree(s, s->sg); s->sg = NULL;
-    for (int q = 0; q < AWP_MAX_COMP; q++) { dfree(s, s->sgt_file[q]); s->sgt_file[q] = NULL; }
+    drop_graphs(s);
+    set_points_release(s);
     s->npts = npts;
     s->sgt_file_floats = file_floats_of(p, npts);
     if (npts == 0) return AWP_OK;
@@ -1200,6 +1370,17 @@ extern "C" awp_status awp_set_points(awp_solver *s, int npts, const int *xyz)
         if (e != cudaSuccess) st = set_err(AWP_ERR_CUDA, "sg coefficients: %s", cudaGetErrorString(e));
     }
     return st;
+}
+
+extern "C" awp_status awp_set_points(awp_solver *s, int npts, const int *xyz)
+{
+    NvtxScope nvtx_("awp_set_points");
+    if (!s) return set_err(AWP_ERR_PARAM, "null solver");
+    return with_room(s, [&] {
+        const awp_status st = set_points_once(s, npts, xyz);
+        if (st == AWP_ERR_OOM) set_points_release(s);
+        return st;
+    });
 }
 
 extern "C" int64_t awp_sgt_file_floats(const awp_solver *s) { return s ? s->sgt_file_floats : 0; }
@@ -1316,6 +1497,7 @@ static cudaError_t build_graph(awp_solver *s, int par)
 static awp_status start_if_needed(awp_solver *s)
 {
     if (s->started) return AWP_OK;
+    if (s->lost) return check_alive(s);
     if (!s->media_loaded) return set_err(AWP_ERR_STATE, "media not loaded");
     if (s->staged_on && !s->staged) {
         /* the arrays are fixed from here on: u v w, the stresses, FP32 media */
@@ -1701,6 +1883,7 @@ extern "C" awp_status awp_get_plane(awp_solver *s, int comp, int field, int k, f
     if (field < 0 || field >= AF_R1) return set_err(AWP_ERR_PARAM, "field %d is not a wavefield or stress", field);
     const AwpGeom &g = s->g;
     if (k < 1 || k > g.nz) return set_err(AWP_ERR_PARAM, "level %d outside 1..%d", k, g.nz);
+    if (s->lost) return check_alive(s);
     CU(cudaSetDevice(s->p.device));
     CU(cudaStreamSynchronize(s->stream));
     const float *src = s->comp[cur_buf(s, s->steps_done)][comp].f[field];
@@ -1788,6 +1971,7 @@ extern "C" awp_status awp_set_field(awp_solver *s, int comp, int field, const fl
     const AwpGeom &g = s->g;
     const size_t w = (size_t)(g.nx + 4), rows = (size_t)(g.ny + 4) * (size_t)(g.nz + 4);
     const int type = field >= AF_R1 ? s->rstore : AWP_STORE_F32;
+    s->wrote = 1;
     if (type == AWP_STORE_BFP) return bfp_set(s, comp, field, in);
     uint16_t *tmp = NULL;
     if (type != AWP_STORE_F32) {
@@ -1884,6 +2068,7 @@ extern "C" awp_status awp_checkpoint_write(awp_solver *s, const char *dir)
 {
     NvtxScope nvtx_("awp_checkpoint_write");
     if (!s || !dir) return set_err(AWP_ERR_PARAM, "null argument");
+    if (s->lost) return check_alive(s);
     awp_status st = awp_sync(s);
     if (st != AWP_OK) return st;
     const awp_params *p = &s->p;
@@ -2072,6 +2257,7 @@ extern "C" awp_status awp_reset(awp_solver *s)
     CU(cudaStreamSynchronize(s->stream));
     s->steps_done = 0;
     s->started = 0;
+    s->wrote = 0;
     s->loop_seconds = 0;
     s->loop_steps = 0;
     s->pending = 0;
@@ -2096,11 +2282,13 @@ extern "C" awp_status awp_device_field(awp_solver *s, int comp, int field, float
     if (!s || !ptr) return set_err(AWP_ERR_PARAM, "null argument");
     if (comp < 0 || comp >= s->p.ncomp || field < 0 || field >= AWP_NF_STATE + AM_N)
         return set_err(AWP_ERR_PARAM, "bad component/field");
+    if (s->lost) return check_alive(s);
     CU(cudaSetDevice(s->p.device));
     CU(cudaStreamSynchronize(s->stream));
     *ptr = field < AWP_NF_STATE ? s->comp[cur_buf(s, s->steps_done)][comp].f[field]
                                 : (float *)s->mdt.m[field - AWP_NF_STATE];
     if (layout) *layout = layout_of(s->g);
+    s->lent = 1;
     return AWP_OK;
 }
 
@@ -2206,6 +2394,7 @@ extern "C" awp_status awp_field_energy_noalloc(const float *const *fields, int n
 extern "C" awp_status awp_energy(awp_solver *s, double *out)
 {
     if (!s || !out) return set_err(AWP_ERR_PARAM, "null argument");
+    if (s->lost) return check_alive(s);
     CU(cudaSetDevice(s->p.device));
     AwpEnergyArgs a;
     energy_args(s, a);
@@ -2218,15 +2407,6 @@ extern "C" awp_status awp_energy(awp_solver *s, double *out)
 /* ------------------------------------------------------------------ */
 /* launch shapes and the autotuner                                     */
 /* ------------------------------------------------------------------ */
-
-static void drop_graphs(awp_solver *s)
-{
-    for (int b = 0; b < 2; b++)
-        if (s->graph[b]) {
-            cudaGraphExecDestroy(s->graph[b]);
-            s->graph[b] = NULL;
-        }
-}
 
 extern "C" awp_status awp_get_tuning(awp_solver *s, awp_tuning *t)
 {

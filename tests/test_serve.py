@@ -107,3 +107,15 @@ def test_configure_rejects_unknown_policy():
         with pytest.raises(awpsgt.AwpError) as e:
             sv.lib.awp_server_configure(sv.h, 7, 0.0, 0.0) and awpsgt._check(sv.lib.awp_server_configure(sv.h, 7, 0.0, 0.0))
         assert e.value.status == 2
+
+
+def test_row_padding_costs_no_residency():
+    """A request's rows are padded only where as many of its size fit in the
+    budget all the same; a budget that held two before holds two."""
+    r = make_request(11, (100, 60, 40), (1, 2), 40)
+    need = awpsgt.footprint_bytes(r[0], 40)
+    for budget, padded in ((2 * need, False), (need, False), (8 * need, True)):
+        with awpsgt.Server(hbm_budget=budget, max_active=2, chunk_steps=20) as sv:
+            info, _ = sv.wait(sv.submit(*r), timeout=600)
+        assert awpsgt.REQ_STATE[info["state"]] == "done"
+        assert (info["footprint"] > need) == padded and info["footprint"] >= need
