@@ -55,7 +55,7 @@ awp_status fail(awp_status st, const char *fmt, ...)
         if (e_ != cudaSuccess) return fail(AWP_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
-constexpr long long SYNTH_ONE_CHUNK = 4000000;   /* trace samples of a batch planned in one chunk */
+constexpr long long SYNTH_ONE_CHUNK = 4000;      /* terms of a batch planned in one chunk at most */
 constexpr int GF_THREADS = 256;
 constexpr int CV_THREADS = 128;
 constexpr int CV_BLOCK = CV_THREADS * 8;   /* output samples of one convolution CTA */
@@ -852,11 +852,15 @@ extern "C" awp_status awp_synth_run(awp_synth *s)
         /* at least four chunks (to overlap the plan with the device) of equal
          * size, none above the term buffer; the first one an eighth of that,
          * so that the device starts while the host plans the rest.  A chunk's
-         * copies, launches and events cost about 30 us, so a batch whose whole
-         * plan takes little more goes in one chunk if it fits: 8 variations of
-         * 72 points (0.4 M trace samples, plan 45 us) 0.39 -> 0.29 ms */
+         * copies, launches and events cost about 30 us, so a small batch goes
+         * in one chunk if it fits.  The plan's time, which the device then
+         * waits for, goes with the terms.  Four chunks against one, ms a run,
+         * outputs of 600 and 2000 samples, slip-rate functions up to 40, 80
+         * and 120, two and three components: 624 terms 0.40-0.45 / 0.29-0.34,
+         * 1368 0.48-0.59 / 0.41-0.54, 2808 0.71-0.96 / 0.68-0.93, 5616
+         * 0.80-1.04 / 0.81-1.09, 11552 1.30-1.77 / 1.41-1.97 */
         long long nch = (total + ucap - 1) / ucap;
-        const bool one = nch <= 1 && total * ntout <= SYNTH_ONE_CHUNK;
+        const bool one = nch <= 1 && total <= SYNTH_ONE_CHUNK;
         nch = one ? 1 : nch < 4 ? 4 : nch;
         const long long full_target = (total + nch - 1) / nch;
         long long target = one ? full_target : (full_target + 7) / 8;
