@@ -856,12 +856,20 @@ awp_status awp_create_rows(const awp_params *pin, int pad, awp_solver **out)
         s->staged_rpt = rpt == 1 || rpt == 2 ? rpt : (p->ncomp == 3 && s->rstore == AWP_STORE_F32 ? 2 : 1);
         s->staged_rpt_vel = env_int("AWP_TUNE_RPTV", 1) == 2 ? 2 : 1;
         /* two or three components share one stress work item (media tiles
-         * and cell coefficients once per level): 14 % faster for fx+fy on
-         * 640 x 640 x 256 (14.7 GB), 3-4 % for fx+fy+fz on 400 x 400 x 200
-         * (6.4 GB), but 10 % slower for fx+fy on 1400 x 1000 x 400 (78 GB),
-         * where one component at a time touches half as many pages at once;
-         * so by default up to 32 GiB of solver state */
-        const int batch_default = (double)awp_footprint_bytes(p, 0) <= 32.0 * (double)(1ull << 30) ? 1 : 0;
+         * and cell coefficients once per level).  Up to 32 GiB of solver state
+         * always: 14 % faster for fx+fy on 640 x 640 x 256 (14.7 GB), 3-4 %
+         * for fx+fy+fz on 400 x 400 x 200 (6.4 GB).  Above, ms a step with one
+         * component per item / side by side: fx+fy 1400 x 1000 x 400 FP32
+         * 44.3 / 37.9, mixed 36.7 / 36.0; 900 x 800 x 600 FP32 34.0 / 28.8;
+         * 1000 x 900 x 500 bf16 32.1 / 31.0; fx+fy+fz 1000 x 900 x 500 bfp
+         * 52.5 / 49.7, mixed 48.7 / 46.9, f16 49.6 / 47.0, elastic 41.1 / 39.3.
+         * The other way round for three components with FP32 memory variables
+         * (51 arrays streamed at once): 1000 x 900 x 500 51.1 / 57.8, 1400 x
+         * 1000 x 400 57.8 / 63.5, 700 x 700 x 400 (38 GiB) 19.5 / 20.4; and
+         * for two elastic ones, 1100 x 900 x 400 20.7 / 21.5. */
+        const bool large = (double)awp_footprint_bytes(p, 0) > 32.0 * (double)(1ull << 30);
+        const bool apart = p->nve == 1 ? p->ncomp == 3 && s->rstore == AWP_STORE_F32 : p->ncomp == 2;
+        const int batch_default = large && apart ? 0 : 1;
         s->staged_batch = env_int("AWP_TUNE_BATCH", batch_default) & 3;
     }
     s->nt_file = nt_file_of(p);

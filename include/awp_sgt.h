@@ -336,8 +336,10 @@ typedef struct {
     int kchunk_sweep;        /* two-sweep stepper: z levels per work item (8..nz)      */
     int staged_batch;        /* staged sweeps with all components of a tile in one work
                                 item, sharing media tiles and cell coefficients:
-                                bit 0 the stress sweep (default 1 up to 32 GiB of
-                                solver state, else 0); bit 1 accepted without effect */
+                                bit 0 the stress sweep (default 1, but 0 above 32 GiB
+                                of solver state for three components with FP32 memory
+                                variables and for two elastic ones); bit 1 accepted
+                                without effect */
     int sm_limit;            /* persistent grids sized for this many SMs (0 = every
                                 SM of the device): solves that share a GPU each take
                                 their share instead of time-slicing the whole device */

@@ -3,9 +3,9 @@ fx+fy+fz stepped together by the default stepper (the staged sweeps, the
 stress sweep with the three components side by side), 5000 SGT points, the
 layered + 5 % perturbed medium; and on the 640x640x256 fx+fy workload the
 same way (two components side by side, 5000 points).  With AWP_FULL_SIZE=1
-also the 1400x1000x400 basin workload, fx+fy, 20000 points, whose FP32
-state (78 GB) puts the default stress sweep on one component per work item;
-it takes about 50 GB of host memory for the oracle and ten minutes, so it is
+also the 1400x1000x400 basin workload, fx+fy, 20000 points, 78 GB of FP32
+state, with the components side by side and with one per work item; each
+takes about 50 GB of host memory for the oracle and ten minutes, so they are
 left out of the regular suite.
 
 The solve starts from a state filled with bounded noise (every wavefield and
@@ -44,9 +44,10 @@ SHAPES = {2: (400, 400, 200, 5000, (1, 2, 3)), 3: (640, 640, 256, 5000, (1, 2)),
 full_size = pytest.mark.skipif(os.environ.get("AWP_FULL_SIZE") != "1", reason="AWP_FULL_SIZE=1 runs it")
 
 
-@pytest.mark.parametrize("config,precision,rstore", [(2, "f32", "f32"), (2, "bfp", "bfp33"), (3, "f32", "f32"),
-                                                     pytest.param(4, "f32", "f32", marks=full_size)])
-def test_workload_bit_exact_from_a_noise_state(config, precision, rstore):
+@pytest.mark.parametrize("config,precision,rstore,batch", [
+    (2, "f32", "f32", 1), (2, "bfp", "bfp33", 1), (3, "f32", "f32", 1),
+    pytest.param(4, "f32", "f32", 0, marks=full_size), pytest.param(4, "f32", "f32", 1, marks=full_size)])
+def test_workload_bit_exact_from_a_noise_state(config, precision, rstore, batch):
     w = ai.config(config)
     media = w.media()
     pts = w.points()
@@ -57,8 +58,8 @@ def test_workload_bit_exact_from_a_noise_state(config, precision, rstore):
     p = awpsgt.make_params(w.nx, w.ny, w.nz, w.dh, w.dt, NT, igreen=w.igreen, nst=NT, precision=precision, **kw)
     with awpsgt.Solver(p) as s:
         tune = s.tuning()
-        # components side by side in the stress sweep up to 32 GiB of state, one per item above
-        assert bool(tune.staged_batch & 1) == (config != 4)
+        tune.staged_batch = batch           # components of the stress sweep side by side (1) or one per item (0)
+        s.set_tuning(tune)
         s.load_media(media)
         for q in range(nc):
             s.set_source(q, [w.src_xyz], stfs[q])
