@@ -139,6 +139,7 @@ def test_autotune_and_cache(kernel, tmp_path):
     # the tuned solve is the oracle's, bit for bit
     small = Case(nx=c.nx, ny=c.ny, nz=c.nz, nt=8, igreen=(1,), srcs=[[(40, 40, 10)]])
     s = solver_for(small, kernel, t)
+    assert s.tuning().as_dict() == t.as_dict()         # the shapes that were timed
     s.run(small.nt)
     assert_same_state(s, small.oracle(0), 0, fields=["u1", "xx", "xy"])
     assert os.path.getsize(cache) > 0
@@ -155,19 +156,18 @@ def test_autotune_rejects_bad_arguments():
 STATE = awpsgt.FIELDS[:15]
 
 
-@pytest.mark.parametrize("batch", [1, 2, 3])
 @pytest.mark.parametrize("igreen", [(1, 2), (1, 2, 3), (-2, 4, 6)])
 @pytest.mark.parametrize("precision", ["f32", "mixed"])
 @pytest.mark.parametrize("nve", [1, 0])
-def test_batched_sweeps_match_per_component(igreen, precision, nve, batch):
-    """Components side by side in one work item (shared media tiles and cell
-    coefficients; batch bit 0 the stress sweep, bit 1 the velocity sweep)
-    against one component per work item: every state field, the CHKJ series
-    and the SGTs bit for bit; FP32 also against the oracle."""
+def test_batched_sweeps_match_per_component(igreen, precision, nve):
+    """Components side by side in one work item of the stress sweep (shared
+    media tiles and cell coefficients) against one component per work item:
+    every state field, the CHKJ series and the SGTs bit for bit; FP32 also
+    against the oracle."""
     n = len(igreen)
     c = Case(nx=45, ny=37, nz=29, nt=30, igreen=igreen, srcs=[[(20, 18, 6)]] * n, nve=nve)
     runs = []
-    for batch in (0, batch):
+    for batch in (0, 1):
         p = awpsgt.make_params(c.nx, c.ny, c.nz, c.dh, c.dt, c.nt, igreen=c.igreen, kernel="staged",
                                precision=precision, **c.kw())
         s = awpsgt.Solver(p)
@@ -189,17 +189,21 @@ def test_batched_sweeps_match_per_component(igreen, precision, nve, batch):
         assert_same_state(b, c.oracle(0), 0, fields=STATE if nve == 1 else STATE[:9])
 
 
-@pytest.mark.parametrize("batch", [0, 1, 3])
-def test_single_level_chunk_all_batch_masks(batch):
-    """nz = 33 in 8-level chunks leaves a one-level chunk at the bottom: the
-    queues of the side-by-side sweeps are set up and rotated on the same
-    level there."""
-    c = Case(nx=40, ny=20, nz=33, nt=20, igreen=(1, 2, 3), srcs=[[(20, 10, 5)], [(21, 9, 6)], [(19, 11, 4)]])
-    s = solver_for(c, "staged", None)
-    s.close()
+@pytest.mark.parametrize("batch", [0, 1])
+@pytest.mark.parametrize("nz,kchunk,sm_limit", [
+    (9, 8, 0), (9, 8, 1),       # chunks of 4 and 5 levels, the shortest an explicit chunk size gives
+    (33, 8, 1),                 # 6 and 7 levels, more items than resident blocks
+    (10, 0, 0),                 # the automatic split's shortest, 5 levels
+    (21, 0, 1),
+])
+def test_short_chunks(nz, kchunk, sm_limit, batch):
+    """The column queues of short chunks, the top one with the free surface
+    included, and rings whose slots and phases carry on from item to item
+    (sm_limit = 1: a few blocks work through all of them)."""
+    c = Case(nx=40, ny=20, nz=nz, nt=20, nd=3, igreen=(1, 2, 3), srcs=[[(20, 10, 5)], [(21, 9, 6)], [(19, 11, 4)]])
     p = awpsgt.make_params(c.nx, c.ny, c.nz, c.dh, c.dt, c.nt, igreen=c.igreen, kernel="staged", **c.kw())
     s = awpsgt.Solver(p)
-    s.set_tuning(variant(s.tuning(), staged_batch=batch, kchunk_staged=8))
+    s.set_tuning(variant(s.tuning(), staged_batch=batch, kchunk_staged=kchunk, sm_limit=sm_limit))
     s.load_media(c.media)
     for q in range(3):
         s.set_source(q, c.srcs[q], c.stfs[q])
@@ -228,32 +232,15 @@ def test_sm_limit_is_bit_exact(kernel):
     s.close()
 
 
-@pytest.mark.parametrize("precision", ["f32", "mixed"])
-def test_generic_ring_loads_are_bit_exact(monkeypatch, precision):
-    """AWP_TUNE_GENERIC=1 (the default above 32 GiB of state) makes the
-    one-component staged sweeps read their rings with generic loads: same
-    arithmetic, so the same bits as the default sweeps and, in FP32, as the
-    oracle."""
-    c = Case(nx=45, ny=37, nz=29, nt=30, igreen=(1, 2), srcs=[[(20, 18, 6)], [(22, 16, 9)]])
-    runs = []
-    for gen in ("0", "1"):
-        monkeypatch.setenv("AWP_TUNE_GENERIC", gen)
-        p = awpsgt.make_params(c.nx, c.ny, c.nz, c.dh, c.dt, c.nt, igreen=c.igreen, kernel="staged",
-                               precision=precision, **c.kw())
-        s = awpsgt.Solver(p)
-        s.set_tuning(variant(s.tuning(), staged_batch=0, kchunk_staged=11))
-        s.load_media(c.media)
-        for q in range(2):
-            s.set_source(q, c.srcs[q], c.stfs[q])
-        s.set_points(c.pts)
-        s.run(c.nt)
-        runs.append(s)
-    a, b = runs
+def test_knobs_of_removed_forms_are_accepted(monkeypatch):
+    """AWP_TUNE_RPTV, bit 1 of AWP_TUNE_BATCH and AWP_TUNE_GENERIC chose forms
+    of the sweeps that are gone: they are taken, reported and change nothing."""
+    for name, value in (("AWP_TUNE_RPTV", "2"), ("AWP_TUNE_BATCH", "3"), ("AWP_TUNE_GENERIC", "1")):
+        monkeypatch.setenv(name, value)
+    c = Case(nx=45, ny=37, nz=29, nt=20, igreen=(1, 2), srcs=[[(20, 18, 6)], [(22, 16, 9)]])
+    s = solver_for(c, "staged")
+    assert s.tuning().staged_rpt_vel == 2 and s.tuning().staged_batch == 3
+    assert "k_vel_tma" in s.profile(1) and "k_str_tmab" in s.profile(1)
+    s.run(c.nt)
     for q in range(2):
-        for f in STATE:
-            assert bits_equal(a.field(f, q), b.field(f, q)), (q, f)
-        assert bits_equal(a.sgt(q), b.sgt(q))
-    if precision == "f32":
-        assert_same_state(b, c.oracle(0), 0)
-    for s in runs:
-        s.close()
+        assert_same_state(s, c.oracle(q), q)
