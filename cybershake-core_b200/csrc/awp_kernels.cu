@@ -506,7 +506,7 @@ k_fused(AwpGeom g, MediaT<TM> md, AwpCompSet<NC> old, AwpCompSet<NC> nw, const f
 /* per-step serial work: source insertion, fstr redo, CHKJ probe       */
 /* ------------------------------------------------------------------ */
 
-/* one warp (step_post.cuh) */
+/* one warp (awp_post.cuh) */
 __global__ void k_post(AwpPostArgs a, int initial) { step_post(a, initial); }
 
 /* SGT gather, pmcl3d.f:1537-1557.  Sample s (0-based) of every point goes
@@ -594,15 +594,13 @@ __global__ void __launch_bounds__(AWP_EN_BLOCK) k_energy_partial(AwpEnergyArgs a
 __global__ void __launch_bounds__(AWP_EN_BLOCK) k_energy_final(const double *partial, int nblocks, int ncomp, double *out,
                                                                int *flag)
 {
-    __shared__ double sh[AWP_EN_GRID * 3];
-    const int n = min(nblocks, AWP_EN_GRID);
-    for (int t = threadIdx.x; t < n * ncomp; t += blockDim.x) sh[t] = partial[t];
+    __shared__ double sh[AWP_EN_GRID * 3];               /* nblocks <= AWP_EN_GRID, ncomp <= 3 */
+    for (int t = threadIdx.x; t < nblocks * ncomp; t += blockDim.x) sh[t] = partial[t];
     __syncthreads();
     const int q = threadIdx.x;
     if (q >= ncomp) return;
     double s = 0.0;
-    for (int b = 0; b < n; ++b) s += sh[b * ncomp + q];
-    for (int b = n; b < nblocks; ++b) s += partial[b * ncomp + q];
+    for (int b = 0; b < nblocks; ++b) s += sh[b * ncomp + q];
     out[q] = s;
     if (flag && !isfinite(s)) atomicExch(flag, 1);
 }

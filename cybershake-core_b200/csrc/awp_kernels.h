@@ -81,7 +81,7 @@ enum { AWP_PART_VEL = 0, AWP_PART_FSVEL = 1, AWP_PART_STR = 2, AWP_PART_FUSED = 
 cudaError_t awp_launch_part(const AwpStepArgs &s, int part, cudaStream_t st);
 /* two-sweep: velocity, free-surface velocity, stress (+ fstr); fused: one kernel */
 cudaError_t awp_launch_step(const AwpStepArgs &s, cudaStream_t st);
-/* TMA-staged sweeps: FP32 media; maps built once over fixed device arrays */
+/* TMA-staged sweeps, every storage of the media; maps built once over fixed device arrays */
 cudaError_t awp_staged_create(AwpStaged **out, const AwpGeom &g, int ncomp, const AwpComp *comp, const AwpMediaT &md,
                               int rtype);
 void awp_staged_destroy(AwpStaged *s);

@@ -514,10 +514,12 @@ static awp_status dalloc(awp_solver *s, void **ptr, size_t bytes)
 }
 
 /* Field arrays.  x = 1 sits at column 8 of a row; the base is placed so that
- * this column starts a 128-byte line (rows are a multiple of 128 bytes,
- * make_geom), so the 32-cell row of a tile is one line of its own instead of
- * parts of two that the neighbouring tile shares.  AWP_TUNE_STAGGER adds that
- * many bytes times the array's ordinal (modulo 32). */
+ * this column of the first row starts a 128-byte line, and with padded rows
+ * (make_geom) that of every row of a 4-byte array: the 32-cell row of a tile
+ * is one line of its own instead of parts of two that the neighbouring tile
+ * shares.  (Rows of a 16-bit array are a multiple of 64 bytes; a tile's row is
+ * half a line.)  AWP_TUNE_STAGGER adds that many bytes times the array's
+ * ordinal (modulo 32). */
 static awp_status dalloc_field(awp_solver *s, void **ptr, size_t bytes, int esize)
 {
     const size_t shift = (size_t)(128 - AWP_XO * esize), off = s->stagger * (size_t)(s->nstag % 32) + shift;
@@ -566,7 +568,8 @@ static awp_status check_params(const awp_params *p)
     if (p->kernel < AWP_KERNEL_AUTO || p->kernel > AWP_KERNEL_STAGED_FMA)
         return set_err(AWP_ERR_PARAM, "unknown kernel %d", p->kernel);
     if ((p->kernel == AWP_KERNEL_STAGED || p->kernel == AWP_KERNEL_STAGED_FMA) && store_of(p) != AWP_STORE_F32)
-        return set_err(AWP_ERR_PARAM, "the staged stepper reads FP32 media (precision f32, mixed or bfp)");
+        return set_err(AWP_ERR_PARAM, "the staged stepper asked for by name takes FP32 media (precision f32, mixed or "
+                       "bfp); kernel auto runs the staged sweeps on 16-bit media");
     if (p->nve == 1 && !(p->fl > 0 && p->fh > p->fl && p->fp > 0)) return set_err(AWP_ERR_PARAM, "Q band needs 0 < FL < FH and FP > 0");
     if (p->npc != 0 && p->npc != 1) return set_err(AWP_ERR_PARAM, "NPC must be 0 (Cerjan) or 1 (PML)");
     if (p->npc == 1) {
@@ -1508,7 +1511,7 @@ static awp_status start_if_needed(awp_solver *s)
     if (s->lost) return check_alive(s);
     if (!s->media_loaded) return set_err(AWP_ERR_STATE, "media not loaded");
     if (s->staged_on && !s->staged) {
-        /* the arrays are fixed from here on: u v w, the stresses, FP32 media */
+        /* the arrays are fixed from here on */
         const cudaError_t e = awp_staged_create(&s->staged, s->g, s->p.ncomp, s->comp[0], s->mdt, s->rstore);
         if (e != cudaSuccess) return set_err(AWP_ERR_CUDA, "staged stepper: tensor maps: %s", cudaGetErrorString(e));
     }

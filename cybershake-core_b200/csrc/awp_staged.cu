@@ -2,15 +2,16 @@
  * awp_staged.cu -- the two-sweep stepper with TMA-staged xy tiles (2.5D blocking).
  *
  * A thread block owns a 32 x 8 column tile (the velocity sweep, awp_pair.cuh:
- * 32 x 16) of one component and marches up a chunk of z levels.  A producer warp issues, for every level, TMA tile loads
- * (cp.async.bulk.tensor over 3D tensor maps of the padded volume) into a ring
- * of shared-memory slots ahead of the level being computed: stencil tiles
- * with a 4-column and 2-row halo, media tiles with the row below, and the
- * point-wise state as 32 x 8 tiles.  A "full" mbarrier per slot counts the
- * bytes in; the eight consumer warps release a slot through its "empty"
- * mbarrier.  Values needed only along the cell's own column (z neighbours)
- * travel in per-thread register queues, loaded one level ahead.  Results are
- * written with coalesced stores.  The bytes in flight per SM are set by the
+ * 32 x 16) and marches up a chunk of z levels, of one component or (stress
+ * sweep) of all of them.  A producer warp issues, for every level, TMA tile
+ * loads (cp.async.bulk.tensor over 3D tensor maps of the padded volume) into a
+ * ring of shared-memory slots ahead of the level being computed: stencil tiles
+ * with a halo, media tiles with the row below, and the point-wise state
+ * without.  A "full" mbarrier per slot counts the bytes in; the consumer warps
+ * release a slot through its "empty" mbarrier.  The stress sweep's values
+ * along the cell's own column (z neighbours) travel in per-thread register
+ * queues, loaded one level ahead; the velocity sweep's come through the ring.
+ * Results are written with coalesced stores.  The bytes in flight per SM are set by the
  * ring depth, not by registers or resident warps.
  *
  * Work items (x tile, y tile, z chunk, component) are spread over a
@@ -277,7 +278,6 @@ __device__ __forceinline__ bool ring_acquire(uint64_t *empty, uint32_t use, cons
 #define STR_ST (3 * ST_VT + 4 * ST_MP)           /* first stress tile        */
 #define STR_SLOT (STR_ST + 12 * ST_PT)           /* r tiles fit in 6 x 256   */
 
-/* media of planes k and k-1 at the cell */
 /* the six stresses of a cell, times the sponge factor, to global memory
  * (the array pointers come from a shared-memory table) */
 __device__ __forceinline__ void gst6(const AwpComp &o, int c, const Stress6 &s, float crj)
@@ -943,7 +943,14 @@ static cudaError_t staged_slots(K kernel, size_t smem, int sm_limit, int threads
  * not outweigh them, and the top chunk's threads mirror the levels nz-2 .. nz
  * themselves.  Steps, fixed 25 .. 40 levels before -> this rule: 100x100x50 one
  * component 0.052 -> 0.037 ms, 160x160x80 0.114 -> 0.084, 120x110x60 two
- * components 0.114 -> 0.072, 400x400x200 three 3.18 -> 3.11. */
+ * components 0.114 -> 0.072, 400x400x200 three 3.18 -> 3.11.
+ * The constants are measured, not derived.  On twelve grids from 64x64x48 to
+ * 640x500x150 with one to three components, 0.65 up to 1.0 gave the same step
+ * to 0.6 %, 0.5 and less cost up to 11 %; extra halved or doubled moved single
+ * grids by 3 %, halved 10 % on one, none at all cost up to 6 %.  Against
+ * explicit chunks of 8, 10, 13, 17, 20, 25, 32 and 40 levels the rule was
+ * within 1.3 % of the best one on every grid; the best single one of them, 8,
+ * was up to 13 % slower. */
 static int pick_chunks(int nz, int tiles, const StagedSlots &sl, double extra)
 {
     const int slots = sl.nsm * sl.per, kmin = nz < 5 ? nz : 5;

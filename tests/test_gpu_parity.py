@@ -233,7 +233,7 @@ def test_mixed_precision_runs_close_to_fp64(precision, kernel):
     measured errors are reported by the error study)."""
     c = Case(nt=80, stf_seed=11)
     if kernel == "staged" and precision != "mixed":
-        # the staged stepper reads FP32 media: asking for it with 16-bit media
+        # by name the staged stepper takes FP32 media: asking for it with 16-bit media
         # is a parameter error, not a silent switch to another stepper
         with pytest.raises(awpsgt.AwpError) as e:
             c.gpu(precision=precision, kernel=kernel)
