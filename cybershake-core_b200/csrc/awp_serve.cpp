@@ -124,8 +124,7 @@ void awp_server::end(Req *r, int state, awp_status st)
 awp_status awp_server::build(Req *r)
 {
     awp_solver *s = nullptr;
-    awp_status st = awp_create_rows(&r->rq.params, r->pad, &s);
-    if (st == AWP_ERR_OOM && r->pad) st = awp_create_rows(&r->rq.params, 0, &s);
+    awp_status st = r->pad ? awp_create(&r->rq.params, &s) : awp_create_rows(&r->rq.params, 0, &s);
     if (st == AWP_OK) st = awp_load_media(s, r->rq.media);
     for (int q = 0; q < r->rq.params.ncomp && st == AWP_OK; q++)
         st = awp_set_source(s, q, r->rq.nsrc[q], r->rq.src_xyz[q], r->rq.stf[q]);

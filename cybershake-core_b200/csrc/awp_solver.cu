@@ -439,7 +439,10 @@ static cudaError_t blk_alloc(int dev, void **ptr, size_t bytes)
         blk_trim(dev);
         e = blk_malloc(dev, ptr, bytes);
     }
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess) {
+        cudaGetLastError();               /* returned here; later launches must not report it again */
+        return e;
+    }
     std::lock_guard<std::mutex> lk(g_blk_mu);
     g_blk_live[*ptr] = BlkInfo{dev, bytes};
     return cudaSuccess;

@@ -147,3 +147,22 @@ def test_solve_that_just_fits_runs_without_row_padding(monkeypatch, nx, ny, nz, 
         s.close()
         awpsgt.release_cached_memory()
     assert awpsgt.device_memory(0) == (live0, 0)
+
+
+def test_solver_goes_on_after_a_refused_allocation():
+    """SGT images of 7 TB: cudaMalloc refuses them at once.  The call reports
+    it, and the solver (its rows no longer padded) and later launches are not
+    affected by the error."""
+    c = Case(nx=100, ny=40, nz=32, nt=30, srcs=[[(50, 20, 10)]])
+    p = awpsgt.make_params(c.nx, c.ny, c.nz, c.dh, c.dt, 300000, igreen=c.igreen,
+                           **dict(c.kw(), nst=c.nt, ntiskp_sgt=1, write_step=10))
+    s = awpsgt.Solver(p)
+    s.load_media(c.media)
+    s.set_source(0, c.srcs[0], c.stfs[0])
+    with pytest.raises(awpsgt.AwpError) as e:
+        s.set_points(np.ones((1000000, 3), np.int32))
+    assert awpsgt.STATUS[e.value.status] == "AWP_ERR_OOM"
+    s.run(c.nt)
+    ref = c.gpu()
+    for f in ("u1", "xx", "xy", "r4"):
+        assert np.array_equal(s.field(f).view(np.uint32), ref.field(f).view(np.uint32)), f
