@@ -639,20 +639,26 @@ static awp_status narrow_rows(awp_solver *s)
         std::vector<void **> refs;                /* where the solver keeps the pointer */
     };
     std::vector<Array> old;
-    for (int wave = 0; wave < 2; wave++)          /* media first */
-        for (int k = 0; k < AWP_MAX_FIELDS; k++) {
-            if (!s->stag[k].raw) continue;
-            Array a{s->stag[k].user, s->stag[k].raw, s->stag[k].esize, 1, {}};
-            for (int m = 0; m < AM_N; m++) {
-                if (s->md.m[m] == a.user) a.wave = 0, a.refs.push_back((void **)&s->md.m[m]);
-                if (s->mdt.m[m] == a.user) a.wave = 0, a.refs.push_back(&s->mdt.m[m]);
+    std::vector<int> idx;
+    try {
+        idx.resize((size_t)s->npts);
+        for (int wave = 0; wave < 2; wave++)      /* media first */
+            for (int k = 0; k < AWP_MAX_FIELDS; k++) {
+                if (!s->stag[k].raw) continue;
+                Array a{s->stag[k].user, s->stag[k].raw, s->stag[k].esize, 1, {}};
+                for (int m = 0; m < AM_N; m++) {
+                    if (s->md.m[m] == a.user) a.wave = 0, a.refs.push_back((void **)&s->md.m[m]);
+                    if (s->mdt.m[m] == a.user) a.wave = 0, a.refs.push_back(&s->mdt.m[m]);
+                }
+                for (int b = 0; b < 2; b++)
+                    for (int q = 0; q < AWP_MAX_COMP; q++)
+                        for (int f = 0; f < AWP_NF_ARRAYS; f++)
+                            if (s->comp[b][q].f[f] == a.user) a.refs.push_back((void **)&s->comp[b][q].f[f]);
+                if (a.wave == wave) old.push_back(std::move(a));
             }
-            for (int b = 0; b < 2; b++)
-                for (int q = 0; q < AWP_MAX_COMP; q++)
-                    for (int f = 0; f < AWP_NF_ARRAYS; f++)
-                        if (s->comp[b][q].f[f] == a.user) a.refs.push_back((void **)&s->comp[b][q].f[f]);
-            if (a.wave == wave) old.push_back(a);
-        }
+    } catch (const std::bad_alloc &) {
+        return AWP_ERR_OOM;
+    }
     auto drop = [&](Array &a) {
         for (int k = 0; k < AWP_MAX_FIELDS; k++)
             if (s->stag[k].raw == a.raw) s->stag[k].raw = NULL;
@@ -684,7 +690,6 @@ static awp_status narrow_rows(awp_solver *s)
     for (int q = 0; q < s->p.ncomp; q++) s->pml_args.comp[q] = s->comp[0][q];
     if (s->p.npc == 1) awp_pml_boxes(s->pml_args);
     if (s->npts > 0) {
-        std::vector<int> idx((size_t)s->npts);
         if (e == cudaSuccess) e = cudaMemcpy(idx.data(), s->pt_idx, sizeof(int) * idx.size(), cudaMemcpyDeviceToHost);
         for (int &c : idx) c = c / o.px * g.px + c % o.px;       /* planes have the same number of rows */
         if (e == cudaSuccess) e = cudaMemcpy(s->pt_idx, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice);

@@ -166,3 +166,47 @@ def test_solver_goes_on_after_a_refused_allocation():
     ref = c.gpu()
     for f in ("u1", "xx", "xy", "r4"):
         assert np.array_equal(s.field(f).view(np.uint32), ref.field(f).view(np.uint32)), f
+
+
+@pytest.mark.parametrize("how", ["set_field", "device_field"])
+def test_written_fields_survive_the_change_of_rows(monkeypatch, how):
+    """A wavefield set before the SGT images no longer fit keeps its values;
+    after a device pointer has been handed out the arrays stay where they are
+    and the failure is reported."""
+    c = Case(nx=100, ny=60, nz=40, nt=240, igreen=(1,), srcs=[[(50, 30, 10)]])
+    npts = 12000
+    pts = np.stack([np.random.default_rng(5).integers(1, n + 1, npts) for n in (c.nx, c.ny, c.nz)], 1)
+    p = awpsgt.make_params(c.nx, c.ny, c.nz, c.dh, c.dt, c.nt, igreen=c.igreen,
+                           **dict(c.kw(), ntiskp_sgt=1, write_step=10))
+    u = np.random.default_rng(6).standard_normal((c.nz + 4, c.ny + 4, c.nx + 4)).astype(np.float32)
+
+    def solve():
+        s = awpsgt.Solver(p)
+        s.load_media(c.media)
+        s.set_source(0, c.srcs[0], c.stfs[0])
+        if how == "set_field":
+            s.set_field("u1", u, 0)
+        else:
+            device_pitch(s)
+        live = awpsgt.device_memory(0)[0]
+        s.set_points(pts)
+        s.run(10)
+        return s, live
+
+    gc.collect()
+    awpsgt.release_cached_memory()
+    s, live = solve()
+    want, after = [s.field(f) for f in ("u1", "xx", "r1")], awpsgt.device_memory(0)[0]
+    s.close()
+    awpsgt.release_cached_memory()
+    # room for the narrow arrays and the SGT images, less than the padding short of the padded ones
+    monkeypatch.setenv("AWP_TEST_DEVICE_BYTES", str(after - (1 << 20)))
+    if how == "device_field":
+        with pytest.raises(awpsgt.AwpError) as e:
+            solve()
+        assert awpsgt.STATUS[e.value.status] == "AWP_ERR_OOM"
+        return
+    s, _ = solve()
+    assert device_pitch(s) == 112 and after > live
+    for a, b in zip([s.field(f) for f in ("u1", "xx", "r1")], want):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
